@@ -24,6 +24,7 @@
 // group base B = 2^(goff+J0) + HB uses twiddle (B << l) + (u >> (K-l)) at its
 // local stage l for register slot u (see ct_reg / gs_reg).
 #pragma once
+#include "fp_sched.hpp"
 #include "gf.cuh"
 
 namespace ntt {
@@ -135,27 +136,35 @@ __device__ __forceinline__ void gs_reg(u64 (&v)[1 << K], const TW& tw, u32 B, u6
 // values stay below 4.5q + 1 and multiplier inputs below 2.5q + 1; inverse
 // (GS) values below 3q + 2, multiplier inputs below 3q + 2.
 //
-// Signed twiddles |w| <= (q-1)/2 (FpArT<true>, the library's double tables):
-// |h/q| <= |y|/2, so with c = |y|/q and q < 2^50, |l| <= (c/16) q and
-//   M1 (needs |y| < 2^52):  |r| <= (1/2 + c/8) q,
-//   M2 (needs |y| < 2^53):  |r| <= (1 + c/8) q,
-// and a round of up to four stages needs one normalisation, at its end:
-//   CT from |x| <= q/2 + 1, M1 in every stage: stage outputs below 1.07q,
-//     1.70q, 2.41q, 3.21q; multiplier inputs below 2.41q < 4q.
-//   GS from |x| <= q/2 + 1: stages one to three by M1 (multiplier inputs
-//     below q + 2, 2q + 4, 4q + 8 < 2^52, since an NTT prime below 2^50 has
-//     q = 1 mod 2n with n >= 2^9, so q <= 2^50 - 2^10 + 1), values below
-//     q + 2, 2q + 4, 4q + 8; stage four
-//     by M2 (input below 8q + 16 < 2^53, |r| <= 2q + 2), sums below 8q + 16.
-// Every value stays an exact integer below 2^53, so the results equal the
-// integer path's canonical residues.
+// Signed twiddles |w| <= (q-1)/2 (FpArS, the library's double tables): |h/q|
+// <= |y|/2, so with c = |y|/q and q < 2^50, |l| <= (c/16) q and
+//   M1 (needs |y| < 2^52, c <= 4)      :  |r| <= (1/2 + c/8) q,
+//   M2 (needs |y| < 2^53, c <= 8):           |r| <= (1 + c/8) q.
+// A value therefore stays exact while it is below 8q, whatever its round, and
+// a multiplied value falls back to 2q or less by itself. So the stages are
+// scheduled at compile time from the bound of their inputs (mul_bound,
+// ct_out, gs_sched; in units of q / 1024): each stage takes M1 while its
+// multiplier inputs are below 4q, else M2, and a value is normalised (three
+// operations) only before a sum that could reach 8q, and where a transform
+// ends. Forward (CT): 1.0q -> 1.63, 2.34, 3.13, 4.02, 5.53, 7.2q over six
+// stages, so 16 stages normalise each value three times, the last of them for
+// the output, where one normalisation per round of four and one on load are
+// five. Inverse (GS): sums double, products do not, so each radix slot has a
+// bound of its own and a round of four normalises 4 slots before its third
+// stage and 8 at its end instead of 16. Every value stays an exact integer
+// below 2^53, so the results equal the integer path's canonical residues.
+// The FP64 pipe is what these passes load most (54-71% busy). Measured with
+// this schedule, the scale of the inverse taken on the un-normalised value and
+// the row walks below, before -> after: 64 x 12 towers of 2^16, products and
+// inverse 650 -> 622 us, embedding 425 -> 415 us; phases of 128 products P1 355
+// -> 336, P2 270 -> 247, P3 1510 -> 1456, P4 1036 -> 1012 us.
 constexpr double FP_M1 = 6755399441055744.0;    // 1.5 * 2^52
 constexpr double FP_M2 = 13510798882111488.0;   // 1.5 * 2^53
 
-template <bool SIGNED_TW>
-struct FpArT {
+struct FpBase {
     using T = double;
     double q, qinv;
+    u64 qi;                      // q as an integer
     __device__ __forceinline__ double norm(double z) const {
         const double k = __dsub_rn(__fma_rn(z, qinv, FP_M1), FP_M1);
         return __fma_rn(-k, q, z);
@@ -168,22 +177,34 @@ struct FpArT {
         const double k = __dsub_rn(__fma_rn(h, qinv, M), M);
         return __dadd_rn(__fma_rn(-k, q, h), l);
     }
-    __device__ __forceinline__ double mul(double y, double w) const { return mulq<true>(y, w); }
-    // x < 4q (any lazy residue of the integer kernels)
+    // x < 4q (any lazy residue of the integer kernels) -> normalised
     __device__ __forceinline__ double in(u64 x) const { return norm(u2d(x)); }
-    // normalised z -> canonical [0, q)
-    __device__ __forceinline__ u64 out(double z) const { return d2u(z < 0.0 ? __dadd_rn(z, q) : z); }
+    __device__ __forceinline__ double in_canon(u64 x) const { return u2d(x); }   // x in [0, q)
+    // normalised z -> canonical [0, q): one FP64 addition puts z, biased, into
+    // the low mantissa bits; the sign is fixed on the integer pipes
+    __device__ __forceinline__ u64 out(double z) const {
+        const long long v = __double_as_longlong(__dadd_rn(z, FP_M1)) - 0x4338000000000000ll;
+        return (u64)(v < 0 ? v + (long long)qi : v);
+    }
     __device__ __forceinline__ u64 bits(double z) const { return (u64)__double_as_longlong(z); }
     __device__ __forceinline__ double unbits(u64 b) const { return __longlong_as_double((long long)b); }
-    __device__ __forceinline__ u64 stage_in(u64 x) const { return bits(in(x)); }
-    __device__ __forceinline__ u64 final_out(u64 b) const { return out(unbits(b)); }
-    // final words already canonical: no lazy-range correction needed
+    // residue [0, q) -> signed double in (-q/2, q/2]
+    __device__ __forceinline__ double sgn(u64 x) const {
+        return u2d(x) - (x > (qi >> 1) ? q : 0.0);
+    }
+    // final word of a forward transform (normalised) -> canonical, also where [0, 2q) would do
     __device__ __forceinline__ u64 final_canon(u64 b) const { return out(unbits(b)); }
     __device__ __forceinline__ u64 final_2q(u64 b) const { return out(unbits(b)); }
-    // pass-to-pass intermediates stay in the policy's own representation
-    __device__ __forceinline__ double from_raw(u64 b) const { return unbits(b); }
-    __device__ __forceinline__ u64 to_raw(double z) const { return bits(z); }
+    // any |z| < 8q -> canonical
+    __device__ __forceinline__ u64 canon(double z) const { return out(norm(z)); }
+};
 
+// Unsigned twiddles (the reference's u64 tables converted on load): every
+// round starts and ends normalised (see above); its bounds do not travel.
+struct FpAr : FpBase {
+    __host__ __device__ static constexpr int fwd_out(int, int) { return 0; }
+    __host__ __device__ static constexpr int inv_out(int, int) { return 0; }
+    __device__ __forceinline__ FpAr(double q_, double qinv_, u64 qi_) : FpBase{q_, qinv_, qi_} {}
     template <int K, int L, class TW>
     __device__ __forceinline__ void ct_stage(double (&v)[1 << K], const TW& tw, u32 B) const {
         static_assert(K <= 4, "bounds are proven for rounds of at most four stages");
@@ -197,12 +218,12 @@ struct FpArT {
             for (int o = 0; o < half; ++o) {
                 double& x = v[g * 2 * half + o];
                 double& y = v[g * 2 * half + o + half];
-                const double r = mulq<!SIGNED_TW>(y, w), xx = x;
+                const double r = mulq<true>(y, w), xx = x;
                 x = __dadd_rn(xx, r);
                 y = __dsub_rn(xx, r);
             }
         }
-        if constexpr ((!SIGNED_TW && L % 2 == 1) || L == K - 1) {
+        if constexpr (L % 2 == 1 || L == K - 1) {
 #pragma unroll
             for (int u = 0; u < (1 << K); ++u) v[u] = norm(v[u]);
         }
@@ -212,7 +233,6 @@ struct FpArT {
     __device__ __forceinline__ void gs_stage(double (&v)[1 << K], const TW& tw, u32 B) const {
         static_assert(K <= 4, "bounds are proven for rounds of at most four stages");
         constexpr int half = 1 << (K - 1 - L);
-        constexpr bool EVEN = !SIGNED_TW || (K - 1 - L) >= 3;
         double wr[1 << L];
         tw_run<L>(tw, B << L, wr);
 #pragma unroll
@@ -224,48 +244,117 @@ struct FpArT {
                 double& y = v[g * 2 * half + o + half];
                 const double xx = x, yy = y;
                 x = __dadd_rn(xx, yy);
-                y = mulq<EVEN>(__dsub_rn(xx, yy), w);
+                y = mulq<true>(__dsub_rn(xx, yy), w);
             }
         }
-        if constexpr ((!SIGNED_TW && (K - L) % 2 == 0) || L == 0) {
+        if constexpr ((K - L) % 2 == 0 || L == 0) {
 #pragma unroll
             for (int u = 0; u < (1 << K); ++u) v[u] = norm(v[u]);
         }
         if constexpr (L > 0) gs_stage<K, L - 1>(v, tw, B);
     }
-    template <int K, class TW>
+    template <int K, int BIN, bool END, class TW>
     __device__ __forceinline__ void fwd(double (&v)[1 << K], const TW& tw, u32 B) const { ct_stage<K, 0>(v, tw, B); }
-    template <int K, class TW>
+    template <int K, int BIN, bool END, class TW>
     __device__ __forceinline__ void inv(double (&v)[1 << K], const TW& tw, u32 B) const { gs_stage<K, K - 1>(v, tw, B); }
 };
-// Unsigned twiddles (the reference's u64 tables converted on load).
-using FpAr = FpArT<false>;
-// Signed twiddles in (-q/2, q/2) (the library's double tables).
-using FpArS = FpArT<true>;
+
+// Signed twiddles in (-q/2, q/2) (the library's double tables), scheduled by
+// bounds: BIN = bound of the inputs; END = this round's results are the
+// forward transform's (normalised) / need no bound for a next round (inverse).
+struct FpArS : FpBase {
+    __host__ __device__ static constexpr int fwd_out(int K, int b) { return ct_out(K, b); }
+    __host__ __device__ static constexpr int inv_out(int K, int b) { return gs_sched(K, b).out; }
+    __device__ __forceinline__ FpArS(double q_, double qinv_, u64 qi_) : FpBase{q_, qinv_, qi_} {}
+    template <int K, int L, int BIN, bool END, class TW>
+    __device__ __forceinline__ void ct_stage(double (&v)[1 << K], const TW& tw, u32 B) const {
+        constexpr int half = 1 << (K - 1 - L);
+        constexpr bool PRE = BIN + mul_bound(BIN) > B_LIM;
+        constexpr int b = PRE ? B_NORM : BIN;
+        static_assert(b + mul_bound(b) <= B_LIM, "forward bound");
+        constexpr bool EVEN = b > B_M1;
+        if constexpr (PRE) {
+#pragma unroll
+            for (int u = 0; u < (1 << K); ++u) v[u] = norm(v[u]);
+        }
+        double wr[1 << L];
+        tw_run<L>(tw, B << L, wr);
+#pragma unroll
+        for (int g = 0; g < (1 << L); ++g) {
+            const double w = wr[g];
+#pragma unroll
+            for (int o = 0; o < half; ++o) {
+                double& x = v[g * 2 * half + o];
+                double& y = v[g * 2 * half + o + half];
+                const double r = mulq<EVEN>(y, w), xx = x;
+                x = __dadd_rn(xx, r);
+                y = __dsub_rn(xx, r);
+            }
+        }
+        if constexpr (L + 1 < K) {
+            ct_stage<K, L + 1, b + mul_bound(b), END>(v, tw, B);
+        } else if constexpr (END) {
+#pragma unroll
+            for (int u = 0; u < (1 << K); ++u) v[u] = norm(v[u]);
+        }
+    }
+    template <int K, int L, int BIN, bool END, class TW>
+    __device__ __forceinline__ void gs_stage(double (&v)[1 << K], const TW& tw, u32 B) const {
+        constexpr int s = K - 1 - L, half = 1 << s;
+        constexpr unsigned pre = gs_sched(K, BIN).pre[s], even = gs_sched(K, BIN).even[s], end = gs_sched(K, BIN).end;
+        double wr[1 << L];
+        tw_run<L>(tw, B << L, wr);
+#pragma unroll
+        for (int g = 0; g < (1 << L); ++g) {
+            const double w = wr[g];
+#pragma unroll
+            for (int o = 0; o < half; ++o) {
+                const int i = g * 2 * half + o;
+                double& x = v[i];
+                double& y = v[i + half];
+                if (pre >> i & 1) x = norm(x);
+                if (pre >> (i + half) & 1) y = norm(y);
+                const double xx = x, yy = y, d = __dsub_rn(xx, yy);
+                x = __dadd_rn(xx, yy);
+                y = (even >> i & 1) ? mulq<true>(d, w) : mulq<false>(d, w);
+            }
+        }
+        if constexpr (L > 0) {
+            gs_stage<K, L - 1, BIN, END>(v, tw, B);
+        } else if constexpr (!END) {
+#pragma unroll
+            for (int u = 0; u < (1 << K); ++u)
+                if (end >> u & 1) v[u] = norm(v[u]);
+        }
+    }
+    template <int K, int BIN, bool END, class TW>
+    __device__ __forceinline__ void fwd(double (&v)[1 << K], const TW& tw, u32 B) const {
+        ct_stage<K, 0, BIN, END>(v, tw, B);
+    }
+    template <int K, int BIN, bool END, class TW>
+    __device__ __forceinline__ void inv(double (&v)[1 << K], const TW& tw, u32 B) const {
+        gs_stage<K, K - 1, BIN, END>(v, tw, B);
+    }
+};
 
 // Integer path: the lazy Harvey/Shoup butterflies above, values as-is.
 struct IntAr {
     using T = u64;
     u64 q, two_q;
+    __host__ __device__ static constexpr int fwd_out(int, int) { return 0; }
+    __host__ __device__ static constexpr int inv_out(int, int) { return 0; }
     __device__ __forceinline__ u64 in(u64 x) const { return x; }
-    __device__ __forceinline__ u64 out(u64 x) const { return x; }
+    __device__ __forceinline__ u64 in_canon(u64 x) const { return x; }
     __device__ __forceinline__ u64 bits(u64 x) const { return x; }
     __device__ __forceinline__ u64 unbits(u64 b) const { return b; }
-    __device__ __forceinline__ u64 stage_in(u64 x) const { return x; }
-    __device__ __forceinline__ u64 final_out(u64 b) const { return b; }
     // lazy [0, 4q) -> canonical [0, q), or -> [0, 2q)
     __device__ __forceinline__ u64 final_canon(u64 b) const { return csub(csub(b, two_q), q); }
     __device__ __forceinline__ u64 final_2q(u64 b) const { return csub(b, two_q); }
-    __device__ __forceinline__ u64 from_raw(u64 b) const { return b; }
-    __device__ __forceinline__ u64 to_raw(u64 v) const { return v; }
-    template <int K, class TW>
+    template <int K, int BIN, bool END, class TW>
     __device__ __forceinline__ void fwd(u64 (&v)[1 << K], const TW& tw, u32 B) const { ct_reg<K>(v, tw, B, q, two_q); }
-    template <int K, class TW>
+    template <int K, int BIN, bool END, class TW>
     __device__ __forceinline__ void inv(u64 (&v)[1 << K], const TW& tw, u32 B) const { gs_reg<K>(v, tw, B, q, two_q); }
 };
-
-__host__ __device__ constexpr int cmin(int a, int b) { return a < b ? a : b; }
-__host__ __device__ constexpr int cmax(int a, int b) { return a > b ? a : b; }
 
 // Geometry of the two passes for one LOGN.
 template <int LOGN>
@@ -294,8 +383,8 @@ __device__ __forceinline__ int rowpad(int c) { return c + (c >> 4); }
 
 // ------------------------------------------------------------------ column pass
 // Round (J0, K) over a column tile: thread groups index gi -> (cl, lo, hidx).
-// LD(r, cl) -> u64 and ST(r, cl, v) address tile-local column cl, global row r.
-template <int A, int C, int NT, int J0, int K, bool FWD, class AR, class TW, class LD, class ST>
+// LD(r, cl) -> T and ST(r, cl, v) address tile-local column cl, global row r.
+template <int A, int C, int NT, int J0, int K, bool FWD, int BIN, bool END, class AR, class TW, class LD, class ST>
 __device__ __forceinline__ void col_round(const AR& ar, const TW& tw, LD&& ld, ST&& st) {
     constexpr int SH = A - J0 - K;
     constexpr int GROUPS = ((1 << A) * C) >> K;
@@ -311,53 +400,49 @@ __device__ __forceinline__ void col_round(const AR& ar, const TW& tw, LD&& ld, S
 #pragma unroll
         for (int u = 0; u < (1 << K); ++u) v[u] = ld(hi + (u << SH) + lo, cl);
         const u32 B = (1u << J0) + (u32)hidx;
-        if constexpr (FWD) ar.template fwd<K>(v, tw, B);
-        else ar.template inv<K>(v, tw, B);
+        if constexpr (FWD) ar.template fwd<K, BIN, END>(v, tw, B);
+        else ar.template inv<K, BIN, END>(v, tw, B);
 #pragma unroll
         for (int u = 0; u < (1 << K); ++u) st(hi + (u << SH) + lo, cl, v[u]);
     }
 }
 
-// Forward column pass: stages 0..A-1. First round loads via `ld`, last round
-// stores via `st`; intermediate rounds go through shared memory `sm`.
 // Barrier between rounds: the whole CTA by default; a warp-specialised
 // kernel passes a named barrier over its transform warps.
 struct CtaSync {
     __device__ __forceinline__ void operator()() const { __syncthreads(); }
 };
 
-// `ld` returns u64 residues below 4q; `st` receives the policy's output
-// (IntAr: lazy [0,4q); FpAr: canonical [0,q)), or with RAW_OUT the policy's
-// own word (ar.to_raw), for a following row pass that reads it with RAW_IN.
-template <int A, int C, int NT, int J0, bool RAW_OUT = false, class AR, class TW, class LD, class ST,
-          class SY = CtaSync>
+// Forward column pass: stages 0..A-1. The first round reads the policy's
+// values (bounded by BIN) through `ld`; the last stores the policy's own
+// words (ar.bits) through `st`, for a following row pass; the rounds between
+// go through shared memory `sm`.
+template <int A, int C, int NT, int J0, int BIN, class AR, class TW, class LD, class ST, class SY = CtaSync>
 __device__ __forceinline__ void fwd_col_rounds(u64* sm, const TW& tw, const AR& ar, LD&& ld, ST&& st,
                                                const SY& sync = SY{}) {
     constexpr int K = cmin(4, A - J0);
     constexpr bool FIRST = (J0 == 0);
     constexpr bool LAST = (J0 + K == A);
     using T = typename AR::T;
-    auto gld = [&](int r, int cl) { return ar.in(ld(r, cl)); };
-    auto gst = [&](int r, int cl, T v) {
-        if constexpr (RAW_OUT) st(r, cl, ar.to_raw(v));
-        else st(r, cl, ar.out(v));
-    };
+    auto gst = [&](int r, int cl, T v) { st(r, cl, ar.bits(v)); };
     auto sld = [&](int r, int cl) { return ar.unbits(sm[r * C + cl]); };
     auto sst = [&](int r, int cl, T v) { sm[r * C + cl] = ar.bits(v); };
-    if constexpr (FIRST && LAST) col_round<A, C, NT, J0, K, true>(ar, tw, gld, gst);
-    else if constexpr (FIRST) col_round<A, C, NT, J0, K, true>(ar, tw, gld, sst);
-    else if constexpr (LAST) col_round<A, C, NT, J0, K, true>(ar, tw, sld, gst);
-    else col_round<A, C, NT, J0, K, true>(ar, tw, sld, sst);
+    if constexpr (FIRST && LAST) col_round<A, C, NT, J0, K, true, BIN, false>(ar, tw, ld, gst);
+    else if constexpr (FIRST) col_round<A, C, NT, J0, K, true, BIN, false>(ar, tw, ld, sst);
+    else if constexpr (LAST) col_round<A, C, NT, J0, K, true, BIN, false>(ar, tw, sld, gst);
+    else col_round<A, C, NT, J0, K, true, BIN, false>(ar, tw, sld, sst);
     if constexpr (!LAST) {
         sync();
-        fwd_col_rounds<A, C, NT, J0 + K, RAW_OUT>(sm, tw, ar, ld, st, sync);
+        fwd_col_rounds<A, C, NT, J0 + K, AR::fwd_out(K, BIN)>(sm, tw, ar, ld, st, sync);
     }
 }
 
 // Inverse column pass: stages A-1..0 (GS). Rounds run from the top stage
 // group down; JE is the exclusive end of the current round's stage range.
-// RAW_IN: `ld` returns the policy's own words written by a RAW_OUT row pass.
-template <int A, int C, int NT, int JE, bool RAW_IN = false, class AR, class TW, class LD, class ST>
+// `ld` returns the words of an inverse row pass as the policy's values
+// (bounded by BIN); `st` receives the policy's values (IntAr: [0, 2q);
+// FpArS: below 8q).
+template <int A, int C, int NT, int JE, int BIN, class AR, class TW, class LD, class ST>
 __device__ __forceinline__ void inv_col_rounds(u64* sm, const TW& tw, const AR& ar, LD&& ld, ST&& st) {
     // partition identical to the forward one: rounds [0,4),[4,8),... last ragged
     constexpr int J0 = ((JE - 1) / 4) * 4;
@@ -365,27 +450,22 @@ __device__ __forceinline__ void inv_col_rounds(u64* sm, const TW& tw, const AR& 
     constexpr bool FIRST = (JE == A);
     constexpr bool LAST = (J0 == 0);
     using T = typename AR::T;
-    auto gld = [&](int r, int cl) {
-        if constexpr (RAW_IN) return ar.from_raw(ld(r, cl));
-        else return ar.in(ld(r, cl));
-    };
-    auto gst = [&](int r, int cl, T v) { st(r, cl, ar.out(v)); };
     auto sld = [&](int r, int cl) { return ar.unbits(sm[r * C + cl]); };
     auto sst = [&](int r, int cl, T v) { sm[r * C + cl] = ar.bits(v); };
-    if constexpr (FIRST && LAST) col_round<A, C, NT, J0, K, false>(ar, tw, gld, gst);
-    else if constexpr (FIRST) col_round<A, C, NT, J0, K, false>(ar, tw, gld, sst);
-    else if constexpr (LAST) col_round<A, C, NT, J0, K, false>(ar, tw, sld, gst);
-    else col_round<A, C, NT, J0, K, false>(ar, tw, sld, sst);
+    if constexpr (FIRST && LAST) col_round<A, C, NT, J0, K, false, BIN, true>(ar, tw, ld, st);
+    else if constexpr (FIRST) col_round<A, C, NT, J0, K, false, BIN, false>(ar, tw, ld, sst);
+    else if constexpr (LAST) col_round<A, C, NT, J0, K, false, BIN, true>(ar, tw, sld, st);
+    else col_round<A, C, NT, J0, K, false, BIN, false>(ar, tw, sld, sst);
     if constexpr (!LAST) {
         __syncthreads();
-        inv_col_rounds<A, C, NT, J0, RAW_IN>(sm, tw, ar, ld, st);
+        inv_col_rounds<A, C, NT, J0, AR::inv_out(K, BIN)>(sm, tw, ar, ld, st);
     }
 }
 
 // ------------------------------------------------------------------ row pass
 // Round (J0, K) over a row tile of RB rows; global row of tile row 0 is R0.
 // Twiddle base B = 2^(A+J0) + ((R0+rl) << J0) + hidx.
-template <int A, int RB, int NT, int J0, int K, bool FWD, class AR, class TW, class LD, class ST>
+template <int A, int RB, int NT, int J0, int K, bool FWD, int BIN, bool END, class AR, class TW, class LD, class ST>
 __device__ __forceinline__ void row_round(const AR& ar, const TW& tw, u32 R0, LD&& ld, ST&& st) {
     constexpr int SH = 8 - J0 - K;
     constexpr int GROUPS = (RB * 256) >> K;
@@ -401,8 +481,8 @@ __device__ __forceinline__ void row_round(const AR& ar, const TW& tw, u32 R0, LD
 #pragma unroll
         for (int u = 0; u < (1 << K); ++u) v[u] = ld(rl, cb + (u << SH));
         const u32 B = (1u << (A + J0)) + ((R0 + (u32)rl) << J0) + (u32)hidx;
-        if constexpr (FWD) ar.template fwd<K>(v, tw, B);
-        else ar.template inv<K>(v, tw, B);
+        if constexpr (FWD) ar.template fwd<K, BIN, END>(v, tw, B);
+        else ar.template inv<K, BIN, END>(v, tw, B);
 #pragma unroll
         for (int u = 0; u < (1 << K); ++u) st(rl, cb + (u << SH), v[u]);
     }
@@ -411,104 +491,94 @@ __device__ __forceinline__ void row_round(const AR& ar, const TW& tw, u32 R0, LD
 template <int KMAX, int J0>
 struct RowK { static constexpr int K = cmin(KMAX, 8 - J0); };
 
-// Forward row pass: stages A..A+7, rounds of KMAX. The first round reads with
-// `ld` (u64 below 4q) directly; the last round writes shared memory, and the
-// caller then reads the tile row-contiguously (coalesced) and converts each
-// word with ar.final_out.
-// RAW_IN: `ld` returns the policy's own words written by a RAW_OUT column pass.
-template <int A, int RB, int NT, int KMAX, int J0, bool RAW_IN = false, class AR, class TW, class LD>
+// Forward row pass: stages A..A+7, rounds of KMAX. The first round reads a
+// forward column pass's words as the policy's values (bounded by BIN) with
+// `ld` directly; the last round writes shared memory, and the caller then
+// reads the tile row-contiguously (coalesced) and converts each word with
+// ar.final_canon or ar.final_2q.
+template <int A, int RB, int NT, int KMAX, int J0, int BIN, class AR, class TW, class LD>
 __device__ __forceinline__ void fwd_row_rounds(u64* sm, const TW& tw, u32 R0, const AR& ar, LD&& ld) {
     constexpr int K = RowK<KMAX, J0>::K;
     constexpr bool LAST = (J0 + K == 8);
     constexpr int STR = 256 + 16;
     using T = typename AR::T;
-    auto gld = [&](int rl, int c) {
-        if constexpr (RAW_IN) return ar.from_raw(ld(rl, c));
-        else return ar.in(ld(rl, c));
-    };
     auto sld = [&](int rl, int c) { return ar.unbits(sm[rl * STR + rowpad(c)]); };
     auto sst = [&](int rl, int c, T v) { sm[rl * STR + rowpad(c)] = ar.bits(v); };
-    if constexpr (J0 == 0) row_round<A, RB, NT, J0, K, true>(ar, tw, R0, gld, sst);
-    else row_round<A, RB, NT, J0, K, true>(ar, tw, R0, sld, sst);
+    if constexpr (J0 == 0) row_round<A, RB, NT, J0, K, true, BIN, LAST>(ar, tw, R0, ld, sst);
+    else row_round<A, RB, NT, J0, K, true, BIN, LAST>(ar, tw, R0, sld, sst);
     __syncthreads();
-    if constexpr (!LAST) fwd_row_rounds<A, RB, NT, KMAX, J0 + K, RAW_IN>(sm, tw, R0, ar, ld);
+    if constexpr (!LAST) fwd_row_rounds<A, RB, NT, KMAX, J0 + K, AR::fwd_out(K, BIN)>(sm, tw, R0, ar, ld);
 }
 
 // Inverse row pass: GS stages A+7..A. Input is staged into shared memory
-// (row-contiguous, coalesced) by the caller through ar.stage_in; the last
-// round stores via `st`, which receives the policy's output.
-// RAW_OUT: `st` receives the policy's own words (ar.to_raw) for a following
-// column pass that reads them with RAW_IN.
-template <int A, int RB, int NT, int KMAX, int JE, bool RAW_OUT = false, class AR, class TW, class ST>
+// (row-contiguous, coalesced) by the caller as the policy's words (bounded by
+// BIN); the last round stores the policy's own words via `st`, for a
+// following column pass.
+template <int A, int RB, int NT, int KMAX, int JE, int BIN, class AR, class TW, class ST>
 __device__ __forceinline__ void inv_row_rounds(u64* sm, const TW& tw, u32 R0, const AR& ar, ST&& st) {
     constexpr int J0 = ((JE - 1) / KMAX) * KMAX;
     constexpr int K = JE - J0;
     constexpr bool LAST = (J0 == 0);
     constexpr int STR = 256 + 16;
     using T = typename AR::T;
-    auto gst = [&](int rl, int c, T v) {
-        if constexpr (RAW_OUT) st(rl, c, ar.to_raw(v));
-        else st(rl, c, ar.out(v));
-    };
+    auto gst = [&](int rl, int c, T v) { st(rl, c, ar.bits(v)); };
     auto sld = [&](int rl, int c) { return ar.unbits(sm[rl * STR + rowpad(c)]); };
     auto sst = [&](int rl, int c, T v) { sm[rl * STR + rowpad(c)] = ar.bits(v); };
-    if constexpr (LAST) row_round<A, RB, NT, J0, K, false>(ar, tw, R0, sld, gst);
+    if constexpr (LAST) row_round<A, RB, NT, J0, K, false, BIN, false>(ar, tw, R0, sld, gst);
     else {
-        row_round<A, RB, NT, J0, K, false>(ar, tw, R0, sld, sst);
+        row_round<A, RB, NT, J0, K, false, BIN, false>(ar, tw, R0, sld, sst);
         __syncthreads();
-        inv_row_rounds<A, RB, NT, KMAX, J0, RAW_OUT>(sm, tw, R0, ar, st);
+        inv_row_rounds<A, RB, NT, KMAX, J0, AR::inv_out(K, BIN)>(sm, tw, R0, ar, st);
     }
 }
 
-// Coalesced walks over a row tile (RB rows x 256), 2 words per step so that a
-// warp touches 512 contiguous bytes.
+// Coalesced walks over a row tile (RB rows x 256 = RB*256/NT words per
+// thread, a warp touching 256 contiguous bytes per step): word e of the tile
+// lies at padded shared-memory index si. NT divides 256 or is a multiple of
+// it, so both advance by constants from the thread's first word.
 template <int RB, int NT, class F>
 __device__ __forceinline__ void row_tile_walk(F&& f) {
-#pragma unroll 4
-    for (int e = threadIdx.x; e < RB * 256; e += NT) f(e >> 8, e & 255);
+    constexpr int PER = RB * 256 / NT;
+    static_assert(PER * NT == RB * 256 && NT <= 256 && 256 % NT == 0 && NT % 16 == 0, "walk geometry");
+    const int t = threadIdx.x, ts = rowpad(t);
+#pragma unroll
+    for (int k = 0; k < PER; ++k)
+        f(t + k * NT, ts + (k * NT / 256) * (256 + 16) + rowpad(k * NT % 256));
 }
 
-// Same walk for staging a tile: every load of the thread (RB*256/NT words)
-// is issued before the first conversion and shared-memory store.
+// Same walk for staging a tile: every load of the thread is issued before the
+// first conversion and shared-memory store.
 template <int RB, int NT, class LD, class ST>
 __device__ __forceinline__ void row_tile_stage(LD&& ld, ST&& st) {
     constexpr int PER = RB * 256 / NT;
-    static_assert(PER * NT == RB * 256 && PER <= 16, "stage geometry");
+    static_assert(PER <= 16, "stage geometry");
     u64 v[PER];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        const int e = threadIdx.x + k * NT;
-        v[k] = ld(e >> 8, e & 255);
-    }
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        const int e = threadIdx.x + k * NT;
-        st(e >> 8, e & 255, v[k]);
-    }
+    for (int k = 0; k < PER; ++k) v[k] = ld((int)threadIdx.x + k * NT);
+    int k = 0;
+    row_tile_walk<RB, NT>([&](int e, int si) { st(e, si, v[k++]); });
 }
 
 // Two-operand staging in batches of 8 words per thread: both operands of a
-// batch are loaded before st(rl, c, a, b) combines them.
+// batch are loaded before st(e, si, a, b) combines them.
 template <int RB, int NT, class LDA, class LDB, class ST>
 __device__ __forceinline__ void row_tile_stage2(LDA&& lda, LDB&& ldb, ST&& st) {
     constexpr int PER = RB * 256 / NT;
     constexpr int BT = PER < 8 ? PER : 8;
-    static_assert(PER * NT == RB * 256 && PER % BT == 0, "stage geometry");
+    static_assert(PER % BT == 0, "stage geometry");
+    u64 a[BT], b[BT];
+    int k = 0;
+    row_tile_walk<RB, NT>([&](int e, int si) {
+        if (k % BT == 0) {
 #pragma unroll
-    for (int k0 = 0; k0 < PER; k0 += BT) {
-        u64 a[BT], b[BT];
-#pragma unroll
-        for (int k = 0; k < BT; ++k) {
-            const int e = threadIdx.x + (k0 + k) * NT;
-            a[k] = lda(e >> 8, e & 255);
-            b[k] = ldb(e >> 8, e & 255);
+            for (int j = 0; j < BT; ++j) {
+                a[j] = lda(e + j * NT);
+                b[j] = ldb(e + j * NT);
+            }
         }
-#pragma unroll
-        for (int k = 0; k < BT; ++k) {
-            const int e = threadIdx.x + (k0 + k) * NT;
-            st(e >> 8, e & 255, a[k], b[k]);
-        }
-    }
+        st(e, si, a[k % BT], b[k % BT]);
+        ++k;
+    });
 }
 
 }  // namespace ntt

@@ -117,7 +117,7 @@ __device__ __forceinline__ u64* slot_ptr(const PairDesc& P, u32 slot, int logn) 
 // FP64 (FP = true, towers with q < 2^50) instantiation of a phase kernel.
 template <bool FP>
 __device__ __forceinline__ auto ar_of(const ModC& m) {
-    if constexpr (FP) return ntt::FpArS{ntt::u2d(m.q), qinv_of(m)};
+    if constexpr (FP) return ntt::FpArS{ntt::u2d(m.q), qinv_of(m), m.q};
     else return ntt::IntAr{m.q, m.two_q};
 }
 template <bool FP>
@@ -207,6 +207,20 @@ __device__ __forceinline__ void mac_terms(u64 (&lo)[VB][2], u64 (&hi)[VB][2], co
     }
 }
 
+// Bounds of the transforms' inputs on the FP64 path (units of q / 1024, see
+// ntt.cuh): P1's tensor products of canonical operands stay below 1.25q, P3's
+// converted digits are normalised, canonical or a sum of at most three signed
+// products (0.63q each), P8's prologue is normalised, U is canonical.
+constexpr int P1_IN = 1290, P3_IN = 1930, P8_IN = ntt::B_NORM, P6_IN = ntt::B_CANON;
+template <bool FP>
+__host__ __device__ constexpr int inv_bound(int x0) {
+    return ntt::inv_row_bound<std::conditional_t<FP, ntt::FpArS, ntt::IntAr>>(x0);
+}
+template <bool FP>
+__host__ __device__ constexpr int fwd_bound(int A, int x0) {
+    return ntt::fwd_col_bound<std::conditional_t<FP, ntt::FpArS, ntt::IntAr>>(A, x0);
+}
+
 // ------------------------------------------------------------------ P1
 template <int LOGN, bool FP>
 __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
@@ -222,31 +236,27 @@ __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc*
     u64* X = slot_ptr(P, w.X + i, LOGN) + (size_t)R0 * 256;
     if (P.mode == EMR) {   // d2 = a1 * b1: both operands of a batch loaded before the products
         const size_t o = ((size_t)i << LOGN) + (size_t)R0 * 256;
+        const u64 *a1 = P.in[1] + o, *b1 = P.in[3] + o;
         ntt::row_tile_stage2<G::RB, G::ROW_THREADS>(
-            [&](int rl, int c) { return P.in[1][o + rl * 256 + c]; },
-            [&](int rl, int c) { return P.in[3][o + rl * 256 + c]; },
-            [&](int rl, int c, u64 a, u64 b) {
+            [&](int e) { return a1[e]; }, [&](int e) { return b1[e]; },
+            [&](int, int si, u64 a, u64 b) {
                 u64 v;
-                if constexpr (FP) {   // canonical operands: the product exactly on the FP64 pipe
-                    if (a < m.q && b < m.q) {
-                        const ntt::FpAr ua{ntt::u2d(m.q), qinv_of(m)};
-                        v = ar.bits(ua.norm(ua.mulq<true>(ntt::u2d(a), ntt::u2d(b))));
-                    } else {
-                        v = ar.stage_in(mulmod(a, b, m));
-                    }
+                if constexpr (FP) {   // canonical operands: the product exactly on the FP64 pipe, below 1.25q
+                    if (a < m.q && b < m.q) v = ar.bits(ar.template mulq<true>(ntt::u2d(a), ntt::u2d(b)));
+                    else v = ar.bits(ar.in_canon(mulmod(a, b, m)));
                 } else {
-                    v = ar.stage_in(mulmod(a, b, m));
+                    v = mulmod(a, b, m);
                 }
-                sm[rl * G::ROW_STRIDE + ntt::rowpad(c)] = v;
+                sm[si] = v;
             });
     } else {
         ntt::row_tile_stage<G::RB, G::ROW_THREADS>(
-            [&](int rl, int c) { return digit_src<LOGN>(P, i, (R0 + rl) * 256 + c, m); },
-            [&](int rl, int c, u64 v) { sm[rl * G::ROW_STRIDE + ntt::rowpad(c)] = ar.stage_in(v); });
+            [&](int e) { return digit_src<LOGN>(P, i, R0 * 256 + e, m); },
+            [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in(v)); });
     }
     __syncthreads();
     auto st = [&](int rl, int c, u64 v) { X[rl * 256 + c] = v; };
-    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, true>(sm, twi_of<FP>(D, i, LOGN), R0, ar, st);
+    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, P1_IN>(sm, twi_of<FP>(D, i, LOGN), R0, ar, st);
 }
 
 template <int LOGN, int PATH>
@@ -272,15 +282,17 @@ __device__ __forceinline__ void p2_inv_col_body(const DevCtx& D, const PairDesc*
     const u64 scp = P.mode == RESCALE ? D.ninvp[i] : lv.up_scale_p[i];
     const WsLayout w = ws_layout(P.L, D.K, D.alpha);
     u64* X = slot_ptr(P, w.X + i, LOGN) + c0;
-    auto ld = [&](int r, int cl) { return X[r * 256 + cl]; };
-    if constexpr (FP) {   // the scale as an exact FP64 product (v, sc < q < 2^50), canonical
-        const ntt::FpAr ua{ntt::u2d(m.q), qinv_of(m)};
-        const double scd = ntt::u2d(sc);
-        auto st = [&](int r, int cl, u64 v) { X[r * 256 + cl] = ua.out(ua.norm(ua.mulq<true>(ntt::u2d(v), scd))); };
-        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, true>(sm, twi_of<FP>(D, i, LOGN), ar_of<FP>(m), ld, st);
+    const auto ar = ar_of<FP>(m);
+    auto ld = [&](int r, int cl) { return ar.unbits(X[r * 256 + cl]); };
+    if constexpr (FP) {   // the signed scale as an exact FP64 product, canonical
+        const double scd = ar.sgn(sc);
+        auto st = [&](int r, int cl, double v) { X[r * 256 + cl] = ar.canon(ar.template mulq<true>(v, scd)); };
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, inv_bound<FP>(P1_IN)>(sm, twi_of<FP>(D, i, LOGN), ar, ld,
+                                                                                    st);
     } else {
         auto st = [&](int r, int cl, u64 v) { X[r * 256 + cl] = shoup(v, sc, scp, m.q); };
-        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, true>(sm, twi_of<FP>(D, i, LOGN), ar_of<FP>(m), ld, st);
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, inv_bound<FP>(P1_IN)>(sm, twi_of<FP>(D, i, LOGN), ar, ld,
+                                                                                    st);
     }
 }
 
@@ -313,8 +325,9 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
     u64* Y = slot_ptr(P, w.Y + p * QlP + i, LOGN) + c0;
     // A 50-bit target whose digit has at most three sources, all below 2^50,
     // converts on the FP64 pipe: every term x_s * QHatModp[s][i] is an exact
-    // FP64 modular product of unsigned operands (|r| <= 2q), their sum stays
-    // below 6q < 2^53, and one normalisation gives the canonical residue.
+    // FP64 modular product with the signed constant (|r| <= 0.63q), and the
+    // transform takes their sum as it is (P3_IN).
+    const auto ar = ar_of<FP>(m);
     bool fpc = false;
     if constexpr (FP) {
         fpc = sp <= 3;
@@ -322,48 +335,47 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
     }
     const u64* pool = D.pool + (fpc ? lv.qmpp_off : lv.qmp_off) + (size_t)st0 * QlP + i;
     if (threadIdx.x < sp) {
-        const u64 c = pool[(size_t)threadIdx.x * QlP];
-        cst[threadIdx.x] = fpc ? (u64)__double_as_longlong(ntt::u2d(c)) : c;
+        u64 c = pool[(size_t)threadIdx.x * QlP];
+        if constexpr (FP) c = fpc ? ar.bits(ar.sgn(c)) : c;
+        cst[threadIdx.x] = c;
     }
     __syncthreads();
-    if (fpc) {
-        const ntt::FpAr ua{ntt::u2d(m.q), qinv_of(m)};
+    auto stf = [&](int r, int cl, u64 v) { Y[r * 256 + cl] = v; };
+    auto ld = [&](int r, int cl) { return ar.unbits(sm[r * G::C + cl]); };
+    if constexpr (FP) {
+        if (fpc) {
 #pragma unroll 1
-        for (int k0 = 0; k0 < CS::PER; k0 += CS_VB) {
-            int r[CS_VB], cl[CS_VB];
-            size_t e[CS_VB];
-            ulonglong2 xv[3][CS_VB];
+            for (int k0 = 0; k0 < CS::PER; k0 += CS_VB) {
+                int r[CS_VB], cl[CS_VB];
+                size_t e[CS_VB];
+                ulonglong2 xv[3][CS_VB];
 #pragma unroll
-            for (int b = 0; b < CS_VB; ++b) {
-                CS::pos(k0 + b, r[b], cl[b]);
-                e[b] = (size_t)r[b] * 256 + cl[b];
-            }
-#pragma unroll
-            for (int t = 0; t < 3; ++t)
-                if ((u32)t < sp)
-#pragma unroll
-                    for (int b = 0; b < CS_VB; ++b) xv[t][b] = ld2(X + ((size_t)t << LOGN) + e[b]);
-#pragma unroll
-            for (int b = 0; b < CS_VB; ++b) {
-                double a0 = 0.0, a1 = 0.0;
+                for (int b = 0; b < CS_VB; ++b) {
+                    CS::pos(k0 + b, r[b], cl[b]);
+                    e[b] = (size_t)r[b] * 256 + cl[b];
+                }
 #pragma unroll
                 for (int t = 0; t < 3; ++t)
-                    if ((u32)t < sp) {
-                        const double c = __longlong_as_double((long long)cst[t]);
-                        a0 = __dadd_rn(a0, ua.mulq<true>(ntt::u2d(xv[t][b].x), c));
-                        a1 = __dadd_rn(a1, ua.mulq<true>(ntt::u2d(xv[t][b].y), c));
-                    }
-                ulonglong2 v;
-                v.x = ua.out(ua.norm(a0));
-                v.y = ua.out(ua.norm(a1));
-                *reinterpret_cast<ulonglong2*>(sm + r[b] * G::C + cl[b]) = v;
+                    if ((u32)t < sp)
+#pragma unroll
+                        for (int b = 0; b < CS_VB; ++b) xv[t][b] = ld2(X + ((size_t)t << LOGN) + e[b]);
+#pragma unroll
+                for (int b = 0; b < CS_VB; ++b) {
+                    double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+                    for (int t = 0; t < 3; ++t)
+                        if ((u32)t < sp) {
+                            const double c = __longlong_as_double((long long)cst[t]);
+                            a0 = __dadd_rn(a0, ar.template mulq<false>(ntt::u2d(xv[t][b].x), c));
+                            a1 = __dadd_rn(a1, ar.template mulq<false>(ntt::u2d(xv[t][b].y), c));
+                        }
+                    *reinterpret_cast<double2*>(sm + r[b] * G::C + cl[b]) = make_double2(a0, a1);
+                }
             }
+            __syncthreads();
+            ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P3_IN>(sm, twf_of<FP>(D, qp, LOGN), ar, ld, stf);
+            return;
         }
-        __syncthreads();
-        auto ld = [&](int r, int cl) { return sm[r * G::C + cl]; };
-        auto stf = [&](int r, int cl, u64 v) { Y[r * 256 + cl] = v; };
-        ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(sm, twf_of<FP>(D, qp, LOGN), ar_of<FP>(m), ld, stf);
-        return;
     }
     // conv_i = sum_s x_s * QHatModp[s][i] (ApproxSwitchCRTBasis), lazy in [0, 4q)
 #pragma unroll 1
@@ -380,15 +392,13 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
 #pragma unroll
         for (int b = 0; b < CS_VB; ++b) {
             ulonglong2 v;
-            v.x = conv_reduce(lo[b][0], hi[b][0], m, D.mont_up);
-            v.y = conv_reduce(lo[b][1], hi[b][1], m, D.mont_up);
+            v.x = ar.bits(ar.in(conv_reduce(lo[b][0], hi[b][0], m, D.mont_up)));
+            v.y = ar.bits(ar.in(conv_reduce(lo[b][1], hi[b][1], m, D.mont_up)));
             *reinterpret_cast<ulonglong2*>(sm + r[b] * G::C + cl[b]) = v;
         }
     }
     __syncthreads();
-    auto ld = [&](int r, int cl) { return sm[r * G::C + cl]; };
-    auto stf = [&](int r, int cl, u64 v) { Y[r * 256 + cl] = v; };
-    ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(sm, twf_of<FP>(D, qp, LOGN), ar_of<FP>(m), ld, stf);
+    ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P3_IN>(sm, twf_of<FP>(D, qp, LOGN), ar, ld, stf);
 }
 
 template <int LOGN, int PATH>
@@ -493,15 +503,18 @@ p3ws_modup_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uin
         } else {
             nb_sync(BAR_FULL + b, W::NT);
             u64* Y = slot_ptr(P, w.Y + p * QlP + i, LOGN) + c0;
-            auto ld = [&](int r, int cl) { return buf[r * G::C + cl]; };
             auto stf = [&](int r, int cl, u64 v) { Y[r * 256 + cl] = v; };
             const XformSync xs{(unsigned)W::NC};
-            if (fp)
-                ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(buf, twf_of<true>(D, qp, LOGN),
-                                                                         ar_of<true>(m), ld, stf, xs);
-            else
-                ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(buf, twf_of<false>(D, qp, LOGN),
-                                                                         ar_of<false>(m), ld, stf, xs);
+            if (fp) {
+                const auto ar = ar_of<true>(m);
+                auto ld = [&](int r, int cl) { return ar.in(buf[r * G::C + cl]); };
+                ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P3_IN>(buf, twf_of<true>(D, qp, LOGN), ar, ld, stf,
+                                                                          xs);
+            } else {
+                auto ld = [&](int r, int cl) { return buf[r * G::C + cl]; };
+                ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P3_IN>(buf, twf_of<false>(D, qp, LOGN),
+                                                                          ar_of<false>(m), ld, stf, xs);
+            }
             if (t + 2 * gridDim.x < ntiles) nb_arrive(BAR_EMPTY + b, W::NT);   // a later tile refills b
         }
     }
@@ -522,12 +535,11 @@ __device__ __forceinline__ void p4_modup_fwd_row_body(const DevCtx& D, const Pai
     const ModC m = D.mod[qp];
     const WsLayout w = ws_layout(L, D.K, D.alpha);
     u64* Y = slot_ptr(P, w.Y + p * QlP + i, LOGN) + (size_t)R0 * 256;
-    auto ld = [&](int rl, int c) { return Y[rl * 256 + c]; };
     const auto ar = ar_of<FP>(m);
-    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, true>(sm, twf_of<FP>(D, qp, LOGN), R0, ar, ld);
-    ntt::row_tile_walk<G::RB, G::ROW_THREADS>([&](int rl, int c) {
-        Y[rl * 256 + c] = ar.final_2q(sm[rl * G::ROW_STRIDE + ntt::rowpad(c)]);
-    });
+    auto ld = [&](int rl, int c) { return ar.unbits(Y[rl * 256 + c]); };
+    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, fwd_bound<FP>(G::A, P3_IN)>(sm, twf_of<FP>(D, qp, LOGN), R0,
+                                                                                       ar, ld);
+    ntt::row_tile_walk<G::RB, G::ROW_THREADS>([&](int e, int si) { Y[e] = ar.final_2q(sm[si]); });
 }
 
 template <int LOGN, int PATH>
@@ -776,7 +788,7 @@ p5_mac_fp(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __res
     const ModC m = D.mod[r];
     const u32 dnum = D.dnum;
     const double qd = ntt::u2d(m.q), hq = ntt::u2d(m.q >> 1);
-    const ntt::FpArS ar{qd, qinv_of(m)};
+    const ntt::FpArS ar{qd, qinv_of(m), m.q};
     const u32 pin = r / D.alpha;                  // digit holding tower r
     auto sgn = [&](u64 x) {                       // canonical -> signed double in (-q/2, q/2]
         const double d = ntt::u2d(x);
@@ -1424,7 +1436,7 @@ __device__ __forceinline__ void p5t_consume_fp(const DevCtx& D, const PairDesc* 
     const u32 K = D.K, pin = r / D.alpha;       // digit holding tower r
     const ModC m = D.mod[r];
     const double qd = ntt::u2d(m.q), hq = ntt::u2d(m.q >> 1);
-    const ntt::FpArS ar{qd, qinv_of(m)};
+    const ntt::FpArS ar{qd, qinv_of(m), m.q};
     auto sgn = [&](u64 x) {                     // canonical -> signed double in (-q/2, q/2]
         const double d = ntt::u2d(x);
         return d > hq ? __dsub_rn(d, qd) : d;
@@ -1583,12 +1595,11 @@ __device__ __forceinline__ void p6_moddown_inv_row_body(const DevCtx& D, const P
     const ModC m = D.mod[qp];
     const auto ar = ar_of<FP>(m);
     u64* X = slot_ptr(P, slot, LOGN) + (size_t)R0 * 256;
-    ntt::row_tile_stage<G::RB, G::ROW_THREADS>(
-        [&](int rl, int cc) { return X[rl * 256 + cc]; },
-        [&](int rl, int cc, u64 v) { sm[rl * G::ROW_STRIDE + ntt::rowpad(cc)] = ar.stage_in(v); });
+    ntt::row_tile_stage<G::RB, G::ROW_THREADS>([&](int e) { return X[e]; },
+                                               [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in_canon(v)); });
     __syncthreads();
     auto st = [&](int rl, int cc, u64 v) { X[rl * 256 + cc] = v; };
-    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, true>(sm, twi_of<FP>(D, qp, LOGN), R0, ar, st);
+    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, P6_IN>(sm, twi_of<FP>(D, qp, LOGN), R0, ar, st);
 }
 
 template <int LOGN, int PATH>
@@ -1620,9 +1631,18 @@ __device__ __forceinline__ void p7a_moddown_inv_col_body(const DevCtx& D, const 
     const ModC m = D.mod[qp];
     const u64 sc = D.pdn[t - 1], scp = D.pdnp[t - 1];
     u64* X = slot_ptr(P, w.RP + c * K + (t - 1), LOGN) + c0;
-    auto ld = [&](int r, int cl) { return X[r * 256 + cl]; };
-    auto st = [&](int r, int cl, u64 v) { X[r * 256 + cl] = shoup(v, sc, scp, m.q); };
-    ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, true>(sm, twi_of<FP>(D, qp, LOGN), ar_of<FP>(m), ld, st);
+    const auto ar = ar_of<FP>(m);
+    auto ld = [&](int r, int cl) { return ar.unbits(X[r * 256 + cl]); };
+    if constexpr (FP) {
+        const double scd = ar.sgn(sc);
+        auto st = [&](int r, int cl, double v) { X[r * 256 + cl] = ar.canon(ar.template mulq<true>(v, scd)); };
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, inv_bound<FP>(P6_IN)>(sm, twi_of<FP>(D, qp, LOGN), ar, ld,
+                                                                                    st);
+    } else {
+        auto st = [&](int r, int cl, u64 v) { X[r * 256 + cl] = shoup(v, sc, scp, m.q); };
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, inv_bound<FP>(P6_IN)>(sm, twi_of<FP>(D, qp, LOGN), ar, ld,
+                                                                                    st);
+    }
 }
 
 template <int LOGN, int PATH>
@@ -1660,9 +1680,18 @@ __device__ __forceinline__ void p7b_moddown_inv_col_body(const DevCtx& D, const 
     // round's store, its 16 K dependent loads per thread set the kernel's time
     // on few tiles: 20.9 -> 15.7 us for P7 of one pair at N = 2^15, and
     // 602 -> 514 us for P7 of 128 pairs at N = 2^16.
-    auto ld = [&](int r, int cl) { return U[r * 256 + cl]; };
-    auto st = [&](int r, int cl, u64 v) { sm[r * G::C + cl] = shoup(v, ni, nip, m.q); };
-    ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, true>(sm, twi_of<FP>(D, l, LOGN), ar_of<FP>(m), ld, st);
+    const auto ar = ar_of<FP>(m);
+    auto ld = [&](int r, int cl) { return ar.unbits(U[r * 256 + cl]); };
+    if constexpr (FP) {
+        const double nid = ar.sgn(ni);
+        auto st = [&](int r, int cl, double v) { sm[r * G::C + cl] = ar.canon(ar.template mulq<true>(v, nid)); };
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, inv_bound<FP>(P6_IN)>(sm, twi_of<FP>(D, l, LOGN), ar, ld,
+                                                                                    st);
+    } else {
+        auto st = [&](int r, int cl, u64 v) { sm[r * G::C + cl] = shoup(v, ni, nip, m.q); };
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, inv_bound<FP>(P6_IN)>(sm, twi_of<FP>(D, l, LOGN), ar, ld,
+                                                                                    st);
+    }
     __syncthreads();
 #pragma unroll 1
     for (int k0 = 0; k0 < CS::PER; k0 += CS_VB) {
@@ -1762,9 +1791,10 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
         }
     }
     __syncthreads();
-    auto ld = [&](int r, int cl) { return sm[r * G::C + cl]; };
+    const auto ar = ar_of<FP>(m);
+    auto ld = [&](int r, int cl) { return ar.in(sm[r * G::C + cl]); };
     auto st = [&](int r, int cl, u64 v) { Z[r * 256 + cl] = v; };
-    ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(sm, twf_of<FP>(D, i, LOGN), ar_of<FP>(m), ld, st);
+    ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P8_IN>(sm, twf_of<FP>(D, i, LOGN), ar, ld, st);
 }
 
 template <int LOGN, bool FP>
@@ -1813,9 +1843,10 @@ __device__ __forceinline__ void p9_final_fwd_row_body(const DevCtx& D, const Pai
     const ModC m = D.mod[i];
     const size_t tile0 = (size_t)R0 * 256;
     const u64* Z = slot_ptr(P, w.Z + c * L + i, LOGN) + tile0;
-    auto ld = [&](int rl, int cc) { return Z[rl * 256 + cc]; };
     const auto ar = ar_of<FP>(m);
-    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, true>(sm, twf_of<FP>(D, i, LOGN), R0, ar, ld);
+    auto ld = [&](int rl, int cc) { return ar.unbits(Z[rl * 256 + cc]); };
+    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, fwd_bound<FP>(G::A, P8_IN)>(sm, twf_of<FP>(D, i, LOGN), R0,
+                                                                                       ar, ld);
     const size_t o = ((size_t)i << LOGN) + tile0;
     u64* out = P.out[c] + o;
     const u64* Wt = slot_ptr(P, w.W + c * L + i, LOGN) + tile0;
@@ -1824,10 +1855,9 @@ __device__ __forceinline__ void p9_final_fwd_row_body(const DevCtx& D, const Pai
     // every W (or rescale input) word of the thread is loaded before the sums
     const u64* addend = mode == RESCALE ? P.in[0] + o : Wt;
     ntt::row_tile_stage<G::RB, G::ROW_THREADS>(
-        [&](int rl, int cc) { return addend[rl * 256 + cc]; },
-        [&](int rl, int cc, u64 a) {
-            const int e = rl * 256 + cc;
-            const u64 v = ar.final_canon(sm[rl * G::ROW_STRIDE + ntt::rowpad(cc)]);
+        [&](int e) { return addend[e]; },
+        [&](int e, int si, u64 a) {
+            const u64 v = ar.final_canon(sm[si]);
             u64 r;
             if (mode == RESCALE) {
                 r = csub(shoup(a, s1, s1p, m.q) + v, m.q);

@@ -35,7 +35,7 @@ __device__ __forceinline__ u64 pw_sub(u64 a, u64 b, u64 q) { return a >= b ? a -
 __device__ __forceinline__ u64 pw_mul(u64 a, u64 b, const ModC& m) {
     if (a >= m.q || b >= m.q) return mulmod(reduce64(a, m), reduce64(b, m), m);
     if (fp_tower(m.q)) {
-        const ntt::FpAr ar{ntt::u2d(m.q), qinv_of(m)};
+        const ntt::FpAr ar{ntt::u2d(m.q), qinv_of(m), m.q};
         return ar.out(ar.norm(ar.mulq<true>(ntt::u2d(a), ntt::u2d(b))));
     }
     return mulmod(a, b, m);

@@ -6,6 +6,8 @@
 // jobs x tiles-per-job. Used by the reference ABI (LaunchNTT_CT /
 // LaunchINTT_GS, one job) and by the batched transform entry points.
 #pragma once
+#include <type_traits>
+
 #include "ntt.cuh"
 
 namespace xf {
@@ -44,14 +46,17 @@ __device__ __forceinline__ u64 lift_word(u64 v, u64 q0, u64 q, u64 r64) {
     return (c < 0 && r) ? q - r : r;
 }
 
+// Bound of a forward column pass's inputs: normalised words, or canonical ones (lifted).
+constexpr int COL_IN = ntt::B_CANON;
+
 // Calls f(arith policy, twiddle accessor) for the job's path.
 template <class F>
 __device__ __forceinline__ void with_path(const Job& j, F&& f) {
     if (j.fp) {
         const double qd = ntt::u2d(j.q);
         const double qi = __ddiv_rn(1.0, qd);
-        if (j.twd) f(ntt::FpArS{qd, qi}, ntt::TwD{j.twd});
-        else f(ntt::FpAr{qd, qi}, ntt::TwDConv{j.w});
+        if (j.twd) f(ntt::FpArS{qd, qi, j.q}, ntt::TwD{j.twd});
+        else f(ntt::FpAr{qd, qi, j.q}, ntt::TwDConv{j.w});
         return;
     }
     const ntt::IntAr ar{j.q, 2 * j.q};
@@ -76,10 +81,10 @@ k_fwd_col(const Job* __restrict__ arr, const Job one) {
     const int c0 = (blockIdx.x % G::COL_TILES) * G::C;
     const Job j = get_job<SINGLE>(arr, one, job);
     u64* x = j.x;
-    auto ld = [&](int r, int cl) { return x[r * 256 + c0 + cl]; };
     auto st = [&](int r, int cl, u64 v) { x[r * 256 + c0 + cl] = v; };
     with_path(j, [&](const auto& ar, const auto& tw) {
-        ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(sm, tw, ar, ld, st);
+        auto ld = [&](int r, int cl) { return ar.in(x[r * 256 + c0 + cl]); };
+        ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, COL_IN>(sm, tw, ar, ld, st);
     });
 }
 
@@ -98,10 +103,10 @@ k_fwd_col_lift(const Job* __restrict__ arr) {
     u64* x = j.x;
     const u64* src = j.lift;
     const u64 q0 = j.lift_q0, q = j.q, r64 = j.lift_r64;
-    auto ld = [&](int r, int cl) { return lift_word(__ldg(src + r * 256 + c0 + cl), q0, q, r64); };
     auto st = [&](int r, int cl, u64 v) { x[r * 256 + c0 + cl] = v; };
     with_path(j, [&](const auto& ar, const auto& tw) {
-        ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, true>(sm, tw, ar, ld, st);
+        auto ld = [&](int r, int cl) { return ar.in_canon(lift_word(__ldg(src + r * 256 + c0 + cl), q0, q, r64)); };
+        ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, COL_IN>(sm, tw, ar, ld, st);
     });
 }
 
@@ -114,12 +119,12 @@ k_fwd_row(const Job* __restrict__ arr, const Job one) {
     const u32 R0 = (blockIdx.x % G::ROW_TILES) * G::RB;
     const Job j = get_job<SINGLE>(arr, one, job);
     u64* x = j.x + (size_t)R0 * 256;
-    auto ld = [&](int rl, int c) { return x[rl * 256 + c]; };
     with_path(j, [&](const auto& ar, const auto& tw) {
-        ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, true>(sm, tw, R0, ar, ld);
-        ntt::row_tile_walk<G::RB, G::ROW_THREADS>([&](int rl, int c) {
-            x[rl * 256 + c] = ar.final_canon(sm[rl * G::ROW_STRIDE + ntt::rowpad(c)]);
-        });
+        using AR = std::decay_t<decltype(ar)>;
+        auto ld = [&](int rl, int c) { return ar.unbits(x[rl * 256 + c]); };
+        ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, ntt::fwd_col_bound<AR>(G::A, COL_IN)>(sm, tw, R0, ar,
+                                                                                                     ld);
+        ntt::row_tile_walk<G::RB, G::ROW_THREADS>([&](int e, int si) { x[e] = ar.final_canon(sm[si]); });
     });
 }
 
@@ -134,11 +139,10 @@ k_inv_row(const Job* __restrict__ arr, const Job one) {
     u64* x = j.x + (size_t)R0 * 256;
     auto st = [&](int rl, int c, u64 v) { x[rl * 256 + c] = v; };
     with_path(j, [&](const auto& ar, const auto& tw) {
-        ntt::row_tile_stage<G::RB, G::ROW_THREADS>(
-            [&](int rl, int c) { return x[rl * 256 + c]; },
-            [&](int rl, int c, u64 v) { sm[rl * G::ROW_STRIDE + ntt::rowpad(c)] = ar.stage_in(v); });
+        ntt::row_tile_stage<G::RB, G::ROW_THREADS>([&](int e) { return x[e]; },
+                                                   [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in(v)); });
         __syncthreads();
-        ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, true>(sm, tw, R0, ar, st);
+        ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, ntt::B_NORM>(sm, tw, R0, ar, st);
     });
 }
 
@@ -152,22 +156,30 @@ k_inv_col(const Job* __restrict__ arr, const Job one) {
     const Job j = get_job<SINGLE>(arr, one, job);
     const u64 q = j.q;
     u64* x = j.x;
-    auto ld = [&](int r, int cl) { return x[r * 256 + c0 + cl]; };
     const u64 sc = j.scale, scp = j.scale_p;
-    if (j.fp && sc < q) {   // n^-1 as an exact FP64 product (both operands below q < 2^50)
-        const ntt::FpAr ua{ntt::u2d(q), __ddiv_rn(1.0, ntt::u2d(q))};
-        const double scd = ntt::u2d(sc);
-        auto st = [&](int r, int cl, u64 v) {
-            x[r * 256 + c0 + cl] = ua.out(ua.norm(ua.mulq<true>(ntt::u2d(v), scd)));
-        };
-        with_path(j, [&](const auto& ar, const auto& tw) {
-            ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, true>(sm, tw, ar, ld, st);
-        });
-        return;
-    }
-    auto st = [&](int r, int cl, u64 v) { x[r * 256 + c0 + cl] = shoup(v, sc, scp, q); };
     with_path(j, [&](const auto& ar, const auto& tw) {
-        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, true>(sm, tw, ar, ld, st);
+        using AR = std::decay_t<decltype(ar)>;
+        auto ld = [&](int r, int cl) { return ar.unbits(x[r * 256 + c0 + cl]); };
+        if constexpr (std::is_same_v<typename AR::T, double>) {
+            // n^-1 as an exact FP64 product with the signed constant: below 2q for a value below 8q
+            if (sc < q) {
+                const double scd = ar.sgn(sc);
+                auto st = [&](int r, int cl, double v) {
+                    x[r * 256 + c0 + cl] = ar.canon(ar.template mulq<true>(v, scd));
+                };
+                ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, ntt::inv_row_bound<AR>(ntt::B_NORM)>(sm, tw, ar,
+                                                                                                         ld, st);
+                return;
+            }
+        }
+        auto st = [&](int r, int cl, typename AR::T v) {
+            u64 u;
+            if constexpr (std::is_same_v<typename AR::T, double>) u = ar.canon(v);
+            else u = v;
+            x[r * 256 + c0 + cl] = shoup(u, sc, scp, q);
+        };
+        ntt::inv_col_rounds<G::A, G::C, G::COL_THREADS, G::A, ntt::inv_row_bound<AR>(ntt::B_NORM)>(sm, tw, ar, ld,
+                                                                                                 st);
     });
 }
 
