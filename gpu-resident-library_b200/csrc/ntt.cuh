@@ -369,8 +369,13 @@ struct Geo {
     static constexpr int COL_TILE = R1 * C;
     static constexpr int COL_TILES = COLS / C;
     static constexpr int COL_THREADS = COL_TILE / 16;
-    // row pass: RB rows x 256 (padded rows in shared memory)
-    static constexpr int RB = cmin(R1, 16);
+    // row pass: RB rows x 256 (padded rows in shared memory). Warps own their
+    // rows (below), so the CTA only sets how finely a small grid spreads: eight
+    // rows, eight CTAs per SM, against sixteen rows and four: one product at
+    // N = 2^15 110.0 -> 107.4 us, 128 products unchanged; four rows gave 106.6
+    // and 437 instead of 434 us for 13 mixed operations at N = 2^14.
+    static constexpr int RB = cmin(R1, 8);
+    static constexpr int ROW_MINB = 8;
     static constexpr int ROW_TILE = RB * COLS;
     static constexpr int ROW_TILES = R1 / RB;
     static constexpr int ROW_THREADS = ROW_TILE / 16;
@@ -464,28 +469,31 @@ __device__ __forceinline__ void inv_col_rounds(u64* sm, const TW& tw, const AR& 
 
 // ------------------------------------------------------------------ row pass
 // Round (J0, K) over a row tile of RB rows; global row of tile row 0 is R0.
-// Twiddle base B = 2^(A+J0) + ((R0+rl) << J0) + hidx.
+// Twiddle base B = 2^(A+J0) + ((R0+rl) << J0) + hidx. Thread t works on row
+// t / 16 in every round and in the walks below, so a warp owns two rows from
+// load to store and a row pass needs no barrier between warps: each runs
+// ahead on its own, where a barrier per round had all eight wait for the last
+// (1.1-1.6 barrier stalls per issue). Phases of 128 products with the barriers
+// -> without: P1 336 -> 323, P4 1012 -> 959, P6 393 -> 363, P9 573 -> 541 us.
 template <int A, int RB, int NT, int J0, int K, bool FWD, int BIN, bool END, class AR, class TW, class LD, class ST>
 __device__ __forceinline__ void row_round(const AR& ar, const TW& tw, u32 R0, LD&& ld, ST&& st) {
     constexpr int SH = 8 - J0 - K;
     constexpr int GROUPS = (RB * 256) >> K;
-    static_assert(GROUPS % NT == 0, "groups must divide evenly");
-#pragma unroll 1
-    for (int gi = threadIdx.x; gi < GROUPS; gi += NT) {
-        const int lo = gi & ((1 << SH) - 1);
-        const int rest = gi >> SH;
-        const int hidx = rest & ((1 << J0) - 1);
-        const int rl = rest >> J0;
-        const int cb = (hidx << (8 - J0)) + lo;
-        typename AR::T v[1 << K];
+    static_assert(GROUPS == NT && K == 4, "a thread owns one radix-16 group of its row in every round");
+    const int gi = threadIdx.x;
+    const int lo = gi & ((1 << SH) - 1);
+    const int rest = gi >> SH;
+    const int hidx = rest & ((1 << J0) - 1);
+    const int rl = rest >> J0;
+    const int cb = (hidx << (8 - J0)) + lo;
+    typename AR::T v[1 << K];
 #pragma unroll
-        for (int u = 0; u < (1 << K); ++u) v[u] = ld(rl, cb + (u << SH));
-        const u32 B = (1u << (A + J0)) + ((R0 + (u32)rl) << J0) + (u32)hidx;
-        if constexpr (FWD) ar.template fwd<K, BIN, END>(v, tw, B);
-        else ar.template inv<K, BIN, END>(v, tw, B);
+    for (int u = 0; u < (1 << K); ++u) v[u] = ld(rl, cb + (u << SH));
+    const u32 B = (1u << (A + J0)) + ((R0 + (u32)rl) << J0) + (u32)hidx;
+    if constexpr (FWD) ar.template fwd<K, BIN, END>(v, tw, B);
+    else ar.template inv<K, BIN, END>(v, tw, B);
 #pragma unroll
-        for (int u = 0; u < (1 << K); ++u) st(rl, cb + (u << SH), v[u]);
-    }
+    for (int u = 0; u < (1 << K); ++u) st(rl, cb + (u << SH), v[u]);
 }
 
 template <int KMAX, int J0>
@@ -506,7 +514,7 @@ __device__ __forceinline__ void fwd_row_rounds(u64* sm, const TW& tw, u32 R0, co
     auto sst = [&](int rl, int c, T v) { sm[rl * STR + rowpad(c)] = ar.bits(v); };
     if constexpr (J0 == 0) row_round<A, RB, NT, J0, K, true, BIN, LAST>(ar, tw, R0, ld, sst);
     else row_round<A, RB, NT, J0, K, true, BIN, LAST>(ar, tw, R0, sld, sst);
-    __syncthreads();
+    __syncwarp();
     if constexpr (!LAST) fwd_row_rounds<A, RB, NT, KMAX, J0 + K, AR::fwd_out(K, BIN)>(sm, tw, R0, ar, ld);
 }
 
@@ -527,35 +535,32 @@ __device__ __forceinline__ void inv_row_rounds(u64* sm, const TW& tw, u32 R0, co
     if constexpr (LAST) row_round<A, RB, NT, J0, K, false, BIN, false>(ar, tw, R0, sld, gst);
     else {
         row_round<A, RB, NT, J0, K, false, BIN, false>(ar, tw, R0, sld, sst);
-        __syncthreads();
+        __syncwarp();
         inv_row_rounds<A, RB, NT, KMAX, J0, AR::inv_out(K, BIN)>(sm, tw, R0, ar, st);
     }
 }
 
-// Coalesced walks over a row tile (RB rows x 256 = RB*256/NT words per
-// thread, a warp touching 256 contiguous bytes per step): word e of the tile
-// lies at padded shared-memory index si. NT divides 256 or is a multiple of
-// it, so both advance by constants from the thread's first word.
+// Coalesced walks over a row tile, each warp over its own two rows (16 words
+// per thread, a warp touching 256 contiguous bytes per step): word e of the
+// tile lies at padded shared-memory index si; both advance by constants from
+// the thread's first word.
 template <int RB, int NT, class F>
 __device__ __forceinline__ void row_tile_walk(F&& f) {
-    constexpr int PER = RB * 256 / NT;
-    static_assert(PER * NT == RB * 256 && NT <= 256 && 256 % NT == 0 && NT % 16 == 0, "walk geometry");
-    const int t = threadIdx.x, ts = rowpad(t);
+    static_assert(NT == RB * 16, "two rows per warp");
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int e0 = w * 512 + l, s0 = w * 2 * (256 + 16) + rowpad(l);
 #pragma unroll
-    for (int k = 0; k < PER; ++k)
-        f(t + k * NT, ts + (k * NT / 256) * (256 + 16) + rowpad(k * NT % 256));
+    for (int k = 0; k < 16; ++k) f(e0 + k * 32, s0 + (k / 8) * (256 + 16) + rowpad(k % 8 * 32));
 }
 
 // Same walk for staging a tile: every load of the thread is issued before the
 // first conversion and shared-memory store.
 template <int RB, int NT, class LD, class ST>
 __device__ __forceinline__ void row_tile_stage(LD&& ld, ST&& st) {
-    constexpr int PER = RB * 256 / NT;
-    static_assert(PER <= 16, "stage geometry");
-    u64 v[PER];
-#pragma unroll
-    for (int k = 0; k < PER; ++k) v[k] = ld((int)threadIdx.x + k * NT);
+    u64 v[16];
     int k = 0;
+    row_tile_walk<RB, NT>([&](int e, int) { v[k++] = ld(e); });
+    k = 0;
     row_tile_walk<RB, NT>([&](int e, int si) { st(e, si, v[k++]); });
 }
 
@@ -563,17 +568,15 @@ __device__ __forceinline__ void row_tile_stage(LD&& ld, ST&& st) {
 // batch are loaded before st(e, si, a, b) combines them.
 template <int RB, int NT, class LDA, class LDB, class ST>
 __device__ __forceinline__ void row_tile_stage2(LDA&& lda, LDB&& ldb, ST&& st) {
-    constexpr int PER = RB * 256 / NT;
-    constexpr int BT = PER < 8 ? PER : 8;
-    static_assert(PER % BT == 0, "stage geometry");
+    constexpr int BT = 8;
     u64 a[BT], b[BT];
     int k = 0;
     row_tile_walk<RB, NT>([&](int e, int si) {
         if (k % BT == 0) {
 #pragma unroll
             for (int j = 0; j < BT; ++j) {
-                a[j] = lda(e + j * NT);
-                b[j] = ldb(e + j * NT);
+                a[j] = lda(e + j * 32);
+                b[j] = ldb(e + j * 32);
             }
         }
         st(e, si, a[k % BT], b[k % BT]);

@@ -254,13 +254,13 @@ __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc*
             [&](int e) { return digit_src<LOGN>(P, i, R0 * 256 + e, m); },
             [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in(v)); });
     }
-    __syncthreads();
+    __syncwarp();
     auto st = [&](int rl, int c, u64 v) { X[rl * 256 + c] = v; };
     ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, P1_IN>(sm, twi_of<FP>(D, i, LOGN), R0, ar, st);
 }
 
 template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, 4)
+__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p1_inv_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
@@ -543,7 +543,7 @@ __device__ __forceinline__ void p4_modup_fwd_row_body(const DevCtx& D, const Pai
 }
 
 template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, 4)
+__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p4_modup_fwd_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
@@ -1597,13 +1597,13 @@ __device__ __forceinline__ void p6_moddown_inv_row_body(const DevCtx& D, const P
     u64* X = slot_ptr(P, slot, LOGN) + (size_t)R0 * 256;
     ntt::row_tile_stage<G::RB, G::ROW_THREADS>([&](int e) { return X[e]; },
                                                [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in_canon(v)); });
-    __syncthreads();
+    __syncwarp();
     auto st = [&](int rl, int cc, u64 v) { X[rl * 256 + cc] = v; };
     ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, P6_IN>(sm, twi_of<FP>(D, qp, LOGN), R0, ar, st);
 }
 
 template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, 4)
+__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p6_moddown_inv_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
@@ -1871,7 +1871,7 @@ __device__ __forceinline__ void p9_final_fwd_row_body(const DevCtx& D, const Pai
 }
 
 template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, 4)
+__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p9_final_fwd_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;

@@ -111,7 +111,7 @@ k_fwd_col_lift(const Job* __restrict__ arr) {
 }
 
 template <int LOGN, bool SINGLE>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, 4)
+__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 k_fwd_row(const Job* __restrict__ arr, const Job one) {
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
@@ -129,7 +129,7 @@ k_fwd_row(const Job* __restrict__ arr, const Job one) {
 }
 
 template <int LOGN, bool SINGLE>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, 4)
+__global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 k_inv_row(const Job* __restrict__ arr, const Job one) {
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
@@ -141,7 +141,7 @@ k_inv_row(const Job* __restrict__ arr, const Job one) {
     with_path(j, [&](const auto& ar, const auto& tw) {
         ntt::row_tile_stage<G::RB, G::ROW_THREADS>([&](int e) { return x[e]; },
                                                    [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in(v)); });
-        __syncthreads();
+        __syncwarp();
         ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, ntt::B_NORM>(sm, tw, R0, ar, st);
     });
 }
