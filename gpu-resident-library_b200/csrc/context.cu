@@ -122,6 +122,8 @@ Context::Context(uint32_t n, const std::vector<u64>& Q, const std::vector<u64>& 
     for (u64 p : P) qmaxP = std::max(qmaxP, p);
     dc_.mont_up = ((unsigned __int128)alpha * qmaxQ < ((unsigned __int128)1 << 64)) ? 1u : 0u;
     dc_.mont_down = ((unsigned __int128)K * qmaxP < ((unsigned __int128)1 << 64)) ? 1u : 0u;
+    // P8's sum has the dropped tower's term beside the K special primes'
+    dc_.wrap_down = conv_wrap_ok(K + 1, std::max(qmaxQ, qmaxP)) ? 1u : 0u;
     auto r64mod = [](u64 m) { return hm::mulmod((1ull << 32) % m, (1ull << 32) % m, m); };
 
     // per-level constants

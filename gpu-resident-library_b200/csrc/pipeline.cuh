@@ -183,10 +183,15 @@ __device__ __forceinline__ u64 conv_reduce(u64 lo, u64 hi, const ModC& m, u32 mo
     return mont ? redc_lazy(lo, hi, m) : barrett_lazy(lo, hi, m.q, m.mu_lo, m.mu_hi);
 }
 
-// lo/hi[b][j] += sum_{t < nterms} base[t * stride + e[b] + j] * coef[t] (128-bit).
+// One term of a basis conversion in shared memory: the constant, and its ratio
+// to the target modulus (quotient form below) or its value as a double (P3's
+// FP64 products).
+struct __align__(16) ConvTerm { u64 c; double f; };
+
+// lo/hi[b][j] += sum_{t < nterms} base[t * stride + e[b] + j] * coef[t].c (128-bit).
 template <int VB>
 __device__ __forceinline__ void mac_terms(u64 (&lo)[VB][2], u64 (&hi)[VB][2], const u64* base, size_t stride,
-                                          u32 nterms, const u64* coef, const size_t (&e)[VB]) {
+                                          u32 nterms, const ConvTerm* coef, const size_t (&e)[VB]) {
     for (u32 t0 = 0; t0 < nterms; t0 += 4) {
         ulonglong2 xv[4][VB];
 #pragma unroll
@@ -197,7 +202,7 @@ __device__ __forceinline__ void mac_terms(u64 (&lo)[VB][2], u64 (&hi)[VB][2], co
 #pragma unroll
         for (int tt = 0; tt < 4; ++tt)
             if (t0 + tt < nterms) {
-                const u64 c = coef[t0 + tt];
+                const u64 c = coef[t0 + tt].c;
 #pragma unroll
                 for (int b = 0; b < VB; ++b) {
                     mac_wide(lo[b][0], hi[b][0], xv[tt][b].x, c);
@@ -221,6 +226,79 @@ __host__ __device__ constexpr int fwd_bound(int A, int x0) {
     return ntt::fwd_col_bound<std::conditional_t<FP, ntt::FpArS, ntt::IntAr>>(A, x0);
 }
 
+// Basis conversion into a tower q < 2^50 by an FP64 quotient (P8, where
+// DevCtx::wrap_down). sum_t x_t c_t mod q needs only
+//   r1 = sum_t x_t c_t - K q   (mod 2^64),   K near S = sum_t x_t (c_t / q),
+// as long as r1 fits 64 bits: low 64-bit products on the integer pipes (one
+// wide and two narrow multiplies) and one FMA per term for S on the FP64 pipe.
+// The 128-bit multiply-add of mac_terms takes four wide multiplies and
+// carries (22 issue cycles a term on one scheduler, measured, a wide multiply
+// five of them) and its Montgomery or Barrett step thirty more. Constants are
+// signed, |c_t / q| <= 1/2. Sources below 2^b are rounded to doubles, so S
+// sums n terms with an error of at most 2^(b-54) (n (n+1) / 2 + 5 n / 2); K is
+// S rounded to a multiple of 2^12 (error 2^11). Where conv_wrap_ok admits (n,
+// b), |r1| < 2^13 q < 2^63, and a second step, K2 = r1 / q rounded, leaves
+// |r| <= q/2 + 1, which the transform takes as it is. Measured: P8 of 128
+// products (N = 2^16, four terms) 1078 -> 966 us, of 48 rotations 492 -> 431 us,
+// of 13 mixed operations (N = 2^14, nine terms) 72 -> 65 us. In P3 and P7 the
+// same form gained nothing: their 50-bit sources already go to exact FP64
+// products, and P7's one conversion per component is not what it waits for.
+constexpr double SIGNED_BIAS = 0x1p84 + 0x1p63 + 0x1p52;   // exact (33 bits)
+__device__ __forceinline__ double x2d(u64 x) {   // RN(x), x < 2^63
+    const double h = __hiloint2double(0x45300000, (int)(x >> 32)), l = __hiloint2double(0x43300000, (int)x);
+    return __dadd_rn(__dsub_rn(h, 0x1.00000001p84), l);
+}
+// ConvTerm of the residue c (canonical mod q), negated when NEG.
+template <bool NEG>
+__device__ __forceinline__ ConvTerm conv_term(u64 c, const ModC& m) {
+    long long v = c > (m.q >> 1) ? (long long)c - (long long)m.q : (long long)c;
+    if (NEG) v = -v;
+    return ConvTerm{(u64)v, __dmul_rn((double)v, qinv_of(m))};
+}
+// lo[b][j] += sum_t x c_t mod 2^64, s[b][j] += sum_t x f_t.
+template <int VB>
+__device__ __forceinline__ void quot_terms(u64 (&lo)[VB][2], double (&s)[VB][2], const u64* base, size_t stride,
+                                           u32 nterms, const ConvTerm* ct, const size_t (&e)[VB]) {
+    for (u32 t0 = 0; t0 < nterms; t0 += 4) {
+        ulonglong2 xv[4][VB];
+#pragma unroll
+        for (int tt = 0; tt < 4; ++tt)
+            if (t0 + tt < nterms)
+#pragma unroll
+                for (int b = 0; b < VB; ++b) xv[tt][b] = ld2(base + (t0 + tt) * stride + e[b]);
+#pragma unroll
+        for (int tt = 0; tt < 4; ++tt)
+            if (t0 + tt < nterms) {
+                const ConvTerm c = ct[t0 + tt];
+#pragma unroll
+                for (int b = 0; b < VB; ++b)
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        const u64 x = j ? xv[tt][b].y : xv[tt][b].x;
+                        lo[b][j] += x * c.c;
+                        s[b][j] = __fma_rn(x2d(x), c.f, s[b][j]);
+                    }
+            }
+    }
+}
+struct WrapConv {
+    u64 q;
+    double qinv;
+    __device__ __forceinline__ explicit WrapConv(const ModC& m) : q(m.q), qinv(qinv_of(m)) {}
+    // r = lo - K q, |r| <= q/2 + 1
+    __device__ __forceinline__ long long finish(u64 lo, double s) const {
+        const long long k = __double_as_longlong(__dadd_rn(s, 0x1.8p64)) - 0x43F8000000000000ll;
+        const u64 r1 = lo - (u64)k * (q << 12);
+        const double h = __hiloint2double(0x45300000, (int)(r1 >> 32) ^ (int)0x80000000);
+        const double rd = __dadd_rn(__dsub_rn(h, SIGNED_BIAS),
+                                    __hiloint2double(0x43300000, (int)r1));
+        const int k2 = __double2loint(__fma_rn(rd, qinv, ntt::FP_M1));
+        return (long long)(r1 - (u64)(long long)k2 * q);
+    }
+    __device__ __forceinline__ double finish_d(u64 lo, double s) const {
+        return __dsub_rn(__longlong_as_double(finish(lo, s) + 0x4338000000000000ll), ntt::FP_M1);
+    }
+};
 // ------------------------------------------------------------------ P1
 template <int LOGN, bool FP>
 __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
@@ -311,7 +389,7 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
     using G = ntt::Geo<LOGN>;
     using CS = ColStage<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
-    __shared__ u64 cst[MAXA];
+    __shared__ ConvTerm cst[MAXA];
     const int c0 = tile * G::C;
     const PairDesc& P = pairs[jb.x];
     const u32 L = P.L, K = D.K, QlP = L + K;
@@ -335,9 +413,10 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
     }
     const u64* pool = D.pool + (fpc ? lv.qmpp_off : lv.qmp_off) + (size_t)st0 * QlP + i;
     if (threadIdx.x < sp) {
-        u64 c = pool[(size_t)threadIdx.x * QlP];
-        if constexpr (FP) c = fpc ? ar.bits(ar.sgn(c)) : c;
-        cst[threadIdx.x] = c;
+        const u64 c = pool[(size_t)threadIdx.x * QlP];
+        ConvTerm t{c, 0.0};
+        if constexpr (FP) t.f = fpc ? ar.sgn(c) : 0.0;
+        cst[threadIdx.x] = t;
     }
     __syncthreads();
     auto stf = [&](int r, int cl, u64 v) { Y[r * 256 + cl] = v; };
@@ -365,7 +444,7 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
 #pragma unroll
                     for (int t = 0; t < 3; ++t)
                         if ((u32)t < sp) {
-                            const double c = __longlong_as_double((long long)cst[t]);
+                            const double c = cst[t].f;
                             a0 = __dadd_rn(a0, ar.template mulq<false>(ntt::u2d(xv[t][b].x), c));
                             a1 = __dadd_rn(a1, ar.template mulq<false>(ntt::u2d(xv[t][b].y), c));
                         }
@@ -450,7 +529,7 @@ p3ws_modup_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uin
     using G = ntt::Geo<LOGN>;
     using W = P3WS<LOGN, NP>;
     extern __shared__ __align__(16) u64 sm[];   // [2][COL_TILE]
-    __shared__ u64 cst[2][MAXA];
+    __shared__ ConvTerm cst[2][MAXA];
     const bool conv = threadIdx.x >= W::NC;
     const u32 ctid = threadIdx.x - W::NC;
     u32 k = 0;
@@ -475,7 +554,7 @@ p3ws_modup_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uin
         if (conv) {
             if (k >= 2) nb_sync(BAR_EMPTY + b, W::NT);      // transform warps released buffer b
             const u64* pool = D.pool + lv.qmp_off + (size_t)st0 * QlP + i;
-            if (ctid < sp) cst[b][ctid] = pool[(size_t)ctid * QlP];
+            if (ctid < sp) cst[b][ctid].c = pool[(size_t)ctid * QlP];
             nb_sync(BAR_CONV, NP);
             const u64* X = slot_ptr(P, w.X + st0, LOGN) + c0;
 #pragma unroll 1
@@ -1659,7 +1738,7 @@ __device__ __forceinline__ void p7b_moddown_inv_col_body(const DevCtx& D, const 
     using G = ntt::Geo<LOGN>;
     using CS = ColStage<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
-    __shared__ u64 cl_[gfx::MAXP];
+    __shared__ ConvTerm cl_[gfx::MAXP];
     const int c0 = tile * G::C;
     const PairDesc& P = pairs[jb.x];
     const u32 L = P.L, K = D.K, c = jb.y / (K + 1), l = L - 1;
@@ -1668,7 +1747,7 @@ __device__ __forceinline__ void p7b_moddown_inv_col_body(const DevCtx& D, const 
     if (threadIdx.x < K) {   // PHatModq[j][l] * P^-1 (* 2^64 with mont_down)
         u64 v = mulmod(D.phatmodq[threadIdx.x * D.fullQ + l], D.pinv[l], m);
         if (D.mont_down) v = mulmod(v, r_mod(m), m);
-        cl_[threadIdx.x] = v;
+        cl_[threadIdx.x].c = v;
     }
     __syncthreads();
     const u64 ni = D.ninvu[l], nip = D.ninvup[l];
@@ -1730,7 +1809,7 @@ p7b_moddown_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const ui
 // ------------------------------------------------------------------ P8
 template <int LOGN, u32 MODE, bool FP>
 __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 c, u32 i, int c0, u64* sm,
-                                        const u64* ci) {
+                                        const ConvTerm* ci) {
     using G = ntt::Geo<LOGN>;
     using CS = ColStage<LOGN>;
     const u32 L = P.L, K = D.K, l = L - 1;
@@ -1747,6 +1826,51 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
     const bool larger = q > ql;
     const u64 diff = larger ? q - ql : (ql - q) % q;
     const u64 s2 = lv.s2[i], s2p = lv.s2p[i];
+    const auto ar = ar_of<FP>(m);
+    auto st = [&](int r, int cl, u64 v) { Z[r * 256 + cl] = v; };
+
+    // Quotient form of the whole prologue: sw_i(r) s2 - sum_j x_j PHatModq cm as
+    // one sum. The centred r enters as r s2 + [r > q_l / 2], since s2 = -q_l^-1
+    // makes -q_l s2 one (mod q_i); ci[K] holds s2, ci[0..K) the negated terms.
+    if constexpr (FP) {
+        if (D.wrap_down) {
+            const WrapConv wc(m);
+#pragma unroll 1
+            for (int k0 = 0; k0 < CS::PER; k0 += P8_VB) {
+                int r[P8_VB], cl[P8_VB];
+                size_t e[P8_VB];
+                u64 lo[P8_VB][2] = {};
+                double sq[P8_VB][2] = {};
+                ulonglong2 xr[P8_VB];
+#pragma unroll
+                for (int b = 0; b < P8_VB; ++b) {
+                    CS::pos(k0 + b, r[b], cl[b]);
+                    e[b] = (size_t)r[b] * 256 + cl[b];
+                    if constexpr (MODE == EMR || MODE == RESCALE) xr[b] = ld2(R + e[b]);
+                }
+                if constexpr (MODE != RESCALE) quot_terms<P8_VB>(lo, sq, XP, (size_t)1 << LOGN, K, ci, e);
+#pragma unroll
+                for (int b = 0; b < P8_VB; ++b) {
+                    double v[2];
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        if constexpr (MODE == EMR || MODE == RESCALE) {
+                            const ConvTerm t = ci[K];
+                            const u64 x = j ? xr[b].y : xr[b].x;
+                            lo[b][j] += x * t.c + (x > half ? 1ull : 0ull);
+                            sq[b][j] = __fma_rn(x2d(x), t.f, sq[b][j]);
+                        }
+                        v[j] = wc.finish_d(lo[b][j], sq[b][j]);
+                    }
+                    *reinterpret_cast<double2*>(sm + r[b] * G::C + cl[b]) = make_double2(v[0], v[1]);
+                }
+            }
+            __syncthreads();
+            auto ld = [&](int r, int cl) { return ar.unbits(sm[r * G::C + cl]); };
+            ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P8_IN>(sm, twf_of<FP>(D, i, LOGN), ar, ld, st);
+            return;
+        }
+    }
 
     // v = sw_i(r_l) * s2 - conv'_i * cm, lazy in [0, 4q)
     auto finish = [&](u64 x, u64 lo, u64 hi) -> u64 {
@@ -1791,9 +1915,7 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
         }
     }
     __syncthreads();
-    const auto ar = ar_of<FP>(m);
     auto ld = [&](int r, int cl) { return ar.in(sm[r * G::C + cl]); };
-    auto st = [&](int r, int cl, u64 v) { Z[r * 256 + cl] = v; };
     ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P8_IN>(sm, twf_of<FP>(D, i, LOGN), ar, ld, st);
 }
 
@@ -1801,10 +1923,11 @@ template <int LOGN, bool FP>
 __device__ __forceinline__ void p8_moddown_fwd_col_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
                                               const u32 tile) {
     extern __shared__ __align__(16) u64 sm[];
-    __shared__ u64 ci[gfx::MAXP];
+    __shared__ ConvTerm ci[gfx::MAXP + 1];
     const int c0 = tile * ntt::Geo<LOGN>::C;
     const PairDesc& P = pairs[jb.x];
     const u32 c = jb.y / P.L, i = jb.y % P.L;
+    const bool quot = FP && D.wrap_down;
     if (threadIdx.x < D.K) {
         // PHatModq[j][i] times the combine factor cm (P^-1 * s1 for EvalMult+Rescale,
         // P^-1 otherwise) and, with mont_down, 2^64: the staged sum then reduces
@@ -1812,8 +1935,14 @@ __device__ __forceinline__ void p8_moddown_fwd_col_body(const DevCtx& D, const P
         const ModC mi = D.mod[i];
         const u64 cm = P.mode == EMR ? D.lvl[P.L].ps1[i] : D.pinv[i];
         u64 v = mulmod(D.phatmodq[threadIdx.x * D.fullQ + i], cm, mi);
-        if (D.mont_down) v = mulmod(v, r_mod(mi), mi);
-        ci[threadIdx.x] = v;
+        if (quot) {
+            ci[threadIdx.x] = conv_term<true>(v, mi);
+        } else {
+            if (D.mont_down) v = mulmod(v, r_mod(mi), mi);
+            ci[threadIdx.x] = ConvTerm{v, 0.0};
+        }
+    } else if (quot && threadIdx.x == D.K && (P.mode == EMR || P.mode == RESCALE)) {
+        ci[D.K] = conv_term<false>(D.lvl[P.L].s2[i], D.mod[i]);
     }
     __syncthreads();
     if (P.mode == EMR) p8_body<LOGN, EMR, FP>(D, P, c, i, c0, sm, ci);
