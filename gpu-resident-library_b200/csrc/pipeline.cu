@@ -38,23 +38,27 @@ struct Variant {
     }
     // Phase k of the jobs in segment PATH (P5 and P7 have one integer kernel
     // and are launched by the caller).
-    static void phase(int k, const Plan& p, cudaStream_t s) {
+    static void phase(int k, const Plan& p, cudaStream_t s, bool& after) {
         using G = ntt::Geo<LOGN>;
         const uint32_t cnt = p.job_cnt[k][PATH];
         if (!cnt) return;
         const DevCtx& D = p.dc;
         const PairDesc* pd = p.d_pairs;
         const uint2* J = p.d_jobs + p.job_off[k][PATH];
+        auto run = [&](auto* kernel, unsigned grid, unsigned block, size_t smem) {
+            gfx::chain_launch(kernel, after, grid, block, smem, s, D, pd, J);
+            after = true;
+        };
         switch (k) {
-            case 0: p1_inv_row<LOGN, PATH><<<cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(D, pd, J); break;
-            case 1: p2_inv_col<LOGN, PATH><<<cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(D, pd, J); break;
-            case 2: p3_modup_fwd_col<LOGN, PATH><<<cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(D, pd, J); break;
-            case 3: p4_modup_fwd_row<LOGN, PATH><<<cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(D, pd, J); break;
-            case 5: p6_moddown_inv_row<LOGN, PATH><<<cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(D, pd, J); break;
-            case 6: p7a_moddown_inv_col<LOGN, PATH><<<cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(D, pd, J); break;
-            case NPHASE: p7b_moddown_inv_col<LOGN, PATH><<<cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(D, pd, J); break;
-            case 7: p8_moddown_fwd_col<LOGN, PATH><<<cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(D, pd, J); break;
-            case 8: p9_final_fwd_row<LOGN, PATH><<<cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(D, pd, J); break;
+            case 0: run(p1_inv_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
+            case 1: run(p2_inv_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case 2: run(p3_modup_fwd_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case 3: run(p4_modup_fwd_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
+            case 5: run(p6_moddown_inv_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
+            case 6: run(p7a_moddown_inv_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case NPHASE: run(p7b_moddown_inv_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case 7: run(p8_moddown_fwd_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case 8: run(p9_final_fwd_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
             default: break;
         }
     }
@@ -97,7 +101,7 @@ struct Launcher {
                              P3WS<LOGN, 256>::SMEM);
     }
     template <int PATH>
-    static void p3ws(const Plan& p, cudaStream_t s) {
+    static void p3ws(const Plan& p, cudaStream_t s, bool& after) {
         using G = ntt::Geo<LOGN>;
         const uint32_t cnt = p.job_cnt[2][PATH];
         if (!cnt) return;
@@ -105,36 +109,39 @@ struct Launcher {
         const uint2* J = p.d_jobs + p.job_off[2][PATH];
         if (p.p3_form == 1) {
             const unsigned grid = std::min<unsigned>(ntiles, 2u * (unsigned)sm_count());
-            p3ws_modup_fwd_col<LOGN, PATH, 128, 2><<<grid, P3WS<LOGN, 128>::NT, P3WS<LOGN, 128>::SMEM, s>>>(
-                p.dc, p.d_pairs, J, ntiles);
+            gfx::chain_launch(p3ws_modup_fwd_col<LOGN, PATH, 128, 2>, after, grid, P3WS<LOGN, 128>::NT,
+                              P3WS<LOGN, 128>::SMEM, s, p.dc, p.d_pairs, J, ntiles);
         } else {
             const unsigned grid = std::min<unsigned>(ntiles, (unsigned)sm_count());
-            p3ws_modup_fwd_col<LOGN, PATH, 256, 1><<<grid, P3WS<LOGN, 256>::NT, P3WS<LOGN, 256>::SMEM, s>>>(
-                p.dc, p.d_pairs, J, ntiles);
+            gfx::chain_launch(p3ws_modup_fwd_col<LOGN, PATH, 256, 1>, after, grid, P3WS<LOGN, 256>::NT,
+                              P3WS<LOGN, 256>::SMEM, s, p.dc, p.d_pairs, J, ntiles);
         }
+        after = true;
     }
     // The integer forms of P5 over the first nint key-row jobs.
-    static void launch_p5_int(const Plan& p, cudaStream_t s, uint32_t nint) {
+    static void launch_p5_int(const Plan& p, cudaStream_t s, uint32_t nint, bool& after) {
         constexpr int MAC_TILES = (1 << LOGN) / MAC_TILE;
         const DevCtx& D = p.dc;
         const unsigned grid = nint * MAC_TILES;
+        auto run = [&](auto* kernel, unsigned g, unsigned block, size_t smem) {
+            gfx::chain_launch(kernel, after, g, block, smem, s, D, p.d_pairs, p.d_mac_jobs, p.d_plist);
+            after = true;
+        };
         if (p.p5_form == P5_TMA && mac_tma_ok(D.dnum))
-            p5_mac_tma<LOGN><<<nint * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum), s>>>(
-                D, p.d_pairs, p.d_mac_jobs, p.d_plist);
+            run(p5_mac_tma<LOGN>, nint * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum));
         else if (p.p5_form == P5_ASYNC && mac_async_ok(D.dnum))
-            p5_mac_async<LOGN><<<grid, MACA_NT, maca_smem((int)D.dnum), s>>>(D, p.d_pairs, p.d_mac_jobs,
-                                                                             p.d_plist);
+            run(p5_mac_async<LOGN>, grid, MACA_NT, maca_smem((int)D.dnum));
         else if (p.p5_form == P5_REG256)
-            p5_mac<LOGN, 256><<<grid, 256, mac_smem(D.dnum), s>>>(D, p.d_pairs, p.d_mac_jobs, p.d_plist);
+            run(p5_mac<LOGN, 256>, grid, 256, mac_smem(D.dnum));
         else
-            p5_mac<LOGN, MAC_NT><<<grid, MAC_NT, mac_smem(D.dnum), s>>>(D, p.d_pairs, p.d_mac_jobs,
-                                                                       p.d_plist);
+            run(p5_mac<LOGN, MAC_NT>, grid, MAC_NT, mac_smem(D.dnum));
     }
     static void launch(const Plan& p, cudaStream_t s, unsigned mask) {
         using G = ntt::Geo<LOGN>;
         constexpr int MAC_TILES = (1 << LOGN) / MAC_TILE;
         attrs(p.dc.dnum);
         const DevCtx& D = p.dc;
+        bool after = false;   // a kernel of this call directly before on `s`
         for (int k = 0; k < NPHASE; ++k) {
             if (!(mask >> k & 1)) continue;
             if (k == 4) {
@@ -150,44 +157,47 @@ struct Launcher {
                     cudaEventRecord(p.ev_fork, s);
                     cudaStreamWaitEvent(p.side, p.ev_fork, 0);
                     sf = p.side;
+                    after = false;
                 }
+                const uint4* fj = p.d_mac_jobs + p.job_off[4][1];
+                auto run = [&](auto* kernel, unsigned g, unsigned block, size_t smem) {
+                    gfx::chain_launch(kernel, after, g, block, smem, sf, D, p.d_pairs, fj, p.d_plist);
+                    after = !split;
+                };
                 if (nfp && p.p5_fp_form == 2 && mac_tma_ok(D.dnum))
-                    p5_mac_fp_tma<LOGN, 3><<<nfp * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum, 3), sf>>>(
-                        D, p.d_pairs, p.d_mac_jobs + p.job_off[4][1], p.d_plist);
+                    run(p5_mac_fp_tma<LOGN, 3>, nfp * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum, 3));
                 else if (nfp && p.p5_fp_form == 3 && mac_tma_ok(D.dnum))
-                    p5_mac_fp_tma<LOGN, 2><<<nfp * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum, 2, true), sf>>>(
-                        D, p.d_pairs, p.d_mac_jobs + p.job_off[4][1], p.d_plist);
+                    run(p5_mac_fp_tma<LOGN, 2>, nfp * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum, 2, true));
                 else if (nfp && p.p5_fp_form == 1)
-                    p5_mac_fp<LOGN, 2, 5><<<nfp * MAC_TILES, MACF_NT, mac_smem(D.dnum), sf>>>(
-                        D, p.d_pairs, p.d_mac_jobs + p.job_off[4][1], p.d_plist);
+                    run(p5_mac_fp<LOGN, 2, 5>, nfp * MAC_TILES, MACF_NT, mac_smem(D.dnum));
                 else if (nfp)
-                    p5_mac_fp<LOGN, 4, 4><<<nfp * MAC_TILES, MACF_NT, mac_smem(D.dnum), sf>>>(
-                        D, p.d_pairs, p.d_mac_jobs + p.job_off[4][1], p.d_plist);
+                    run(p5_mac_fp<LOGN, 4, 4>, nfp * MAC_TILES, MACF_NT, mac_smem(D.dnum));
                 if (split) {
-                    launch_p5_int(p, s, nint);
+                    launch_p5_int(p, s, nint, after);
                     cudaEventRecord(p.ev_join, p.side);
                     cudaStreamWaitEvent(s, p.ev_join, 0);
+                    after = false;
                     continue;
                 }
                 if (!nint) continue;
-                launch_p5_int(p, s, nint);
+                launch_p5_int(p, s, nint, after);
             } else if (k == 6) {   // P7a then P7b (U and r_l need the P towers)
                 for (int kk : {6, (int)NPHASE}) {
                     if ((p.mix >> 6 & 1) && p.job_cnt[kk][0] && p.job_cnt[kk][1]) {
-                        Variant<LOGN, 2>::phase(kk, p, s);
+                        Variant<LOGN, 2>::phase(kk, p, s, after);
                     } else {
-                        Variant<LOGN, 0>::phase(kk, p, s);
-                        Variant<LOGN, 1>::phase(kk, p, s);
+                        Variant<LOGN, 0>::phase(kk, p, s, after);
+                        Variant<LOGN, 1>::phase(kk, p, s, after);
                     }
                 }
             } else if (k == 2 && p.p3_form) {
-                if ((p.mix >> 2 & 1) && p.job_cnt[2][0] && p.job_cnt[2][1]) p3ws<2>(p, s);
-                else { p3ws<0>(p, s); p3ws<1>(p, s); }
+                if ((p.mix >> 2 & 1) && p.job_cnt[2][0] && p.job_cnt[2][1]) p3ws<2>(p, s, after);
+                else { p3ws<0>(p, s, after); p3ws<1>(p, s, after); }
             } else if ((p.mix >> k & 1) && p.job_cnt[k][0] && p.job_cnt[k][1]) {
-                Variant<LOGN, 2>::phase(k, p, s);
+                Variant<LOGN, 2>::phase(k, p, s, after);
             } else {
-                Variant<LOGN, 0>::phase(k, p, s);
-                Variant<LOGN, 1>::phase(k, p, s);
+                Variant<LOGN, 0>::phase(k, p, s, after);
+                Variant<LOGN, 1>::phase(k, p, s, after);
             }
         }
     }

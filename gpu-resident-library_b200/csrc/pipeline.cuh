@@ -35,6 +35,7 @@
 
 #include "context.hpp"
 #include "ntt.cuh"
+#include "pdl.cuh"
 
 namespace pl {
 
@@ -340,6 +341,7 @@ __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc*
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p1_inv_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
     on_path<PATH>(jb, [&](auto fp) { p1_inv_row_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -377,6 +379,7 @@ __device__ __forceinline__ void p2_inv_col_body(const DevCtx& D, const PairDesc*
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 p2_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
     on_path<PATH>(jb, [&](auto fp) { p2_inv_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -483,6 +486,7 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 p3_modup_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
     on_path<PATH>(jb, [&](auto fp) { p3_modup_fwd_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -526,6 +530,7 @@ template <int LOGN, int PATH, int NP, int MINB>
 __global__ void __launch_bounds__(P3WS<LOGN, NP>::NT, MINB)
 p3ws_modup_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs,
                    const u32 ntiles) {
+    gfx::chain_begin();
     using G = ntt::Geo<LOGN>;
     using W = P3WS<LOGN, NP>;
     extern __shared__ __align__(16) u64 sm[];   // [2][COL_TILE]
@@ -624,6 +629,7 @@ __device__ __forceinline__ void p4_modup_fwd_row_body(const DevCtx& D, const Pai
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p4_modup_fwd_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
     on_path<PATH>(jb, [&](auto fp) { p4_modup_fwd_row_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -649,6 +655,7 @@ template <int LOGN, int NT>
 __global__ void __launch_bounds__(NT, NT == 128 ? 4 : 3)
 p5_mac(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __restrict__ jobs,
        const u32* __restrict__ plist) {
+    gfx::chain_begin();
     constexpr int TILES = (1 << LOGN) / MAC_TILE;
     constexpr int NV = MAC_TILE / (2 * NT);   // 16-byte vectors per thread
     extern __shared__ __align__(16) u64 sm[];     // [dnum][2][MAC_TILE]
@@ -856,6 +863,7 @@ template <int LOGN, int PCH, int MINB>
 __global__ void __launch_bounds__(MACF_NT, MINB)
 p5_mac_fp(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __restrict__ jobs,
           const u32* __restrict__ plist) {
+    gfx::chain_begin();
     constexpr int NT = MACF_NT;
     constexpr int TILES = (1 << LOGN) / MAC_TILE;
     constexpr int NV = MAC_TILE / (2 * NT);   // 16-byte vectors per thread
@@ -1056,6 +1064,7 @@ template <int LOGN>
 __global__ void __launch_bounds__(MACA_NT)
 p5_mac_async(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __restrict__ jobs,
              const u32* __restrict__ plist) {
+    gfx::chain_begin();
     constexpr int TILES = (1 << LOGN) / MAC_TILE;
     extern __shared__ __align__(16) u64 sm[];   // key [dnum][2][TILE] | stage [2][slots][TILE]
     const uint4 jb = jobs[blockIdx.x / TILES];
@@ -1484,6 +1493,7 @@ template <int LOGN>
 __global__ void __launch_bounds__(P5T_NT)
 p5_mac_tma(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __restrict__ jobs,
            const u32* __restrict__ plist) {
+    gfx::chain_begin();
     constexpr int TILES = (1 << LOGN) / P5T_TILE;
     extern __shared__ __align__(128) u64 sm[];  // mbarriers | key [dnum][2][TILE] | stage [S][slots][TILE]
     const uint4 jb = jobs[blockIdx.x / TILES];
@@ -1644,6 +1654,7 @@ template <int LOGN, int S>
 __global__ void __launch_bounds__(P5T_NT, S == 2 ? 5 : 3)
 p5_mac_fp_tma(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __restrict__ jobs,
               const u32* __restrict__ plist) {
+    gfx::chain_begin();
     constexpr int TILES = (1 << LOGN) / P5T_TILE;
     extern __shared__ __align__(128) u64 sm[];  // mbarriers | key [dnum][2][TILE] | stage [S][slots][TILE]
     const uint4 jb = jobs[blockIdx.x / TILES];
@@ -1684,6 +1695,7 @@ __device__ __forceinline__ void p6_moddown_inv_row_body(const DevCtx& D, const P
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p6_moddown_inv_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
     on_path<PATH>(jb, [&](auto fp) { p6_moddown_inv_row_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -1727,6 +1739,7 @@ __device__ __forceinline__ void p7a_moddown_inv_col_body(const DevCtx& D, const 
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 p7a_moddown_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
     on_path<PATH>(jb, [&](auto fp) { p7a_moddown_inv_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -1801,6 +1814,7 @@ __device__ __forceinline__ void p7b_moddown_inv_col_body(const DevCtx& D, const 
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 p7b_moddown_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
     on_path<PATH>(jb, [&](auto fp) { p7b_moddown_inv_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -1953,6 +1967,7 @@ __device__ __forceinline__ void p8_moddown_fwd_col_body(const DevCtx& D, const P
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 p8_moddown_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
     on_path<PATH>(jb, [&](auto fp) { p8_moddown_fwd_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
@@ -2002,6 +2017,7 @@ __device__ __forceinline__ void p9_final_fwd_row_body(const DevCtx& D, const Pai
 template <int LOGN, int PATH>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 p9_final_fwd_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
+    gfx::chain_begin();
     uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::ROW_TILES];
     const u32 tile = blockIdx.x % ntt::Geo<LOGN>::ROW_TILES;
     on_path<PATH>(jb, [&](auto fp) { p9_final_fwd_row_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });

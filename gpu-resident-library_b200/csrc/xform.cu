@@ -17,12 +17,13 @@ cudaError_t launch_t(const xf::Job* jobs, const xf::Job* one, int njobs, bool in
     const xf::Job o = one ? *one : xf::Job{};
     if (!inverse) {
         xf::k_fwd_col<LOGN, SINGLE><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs, o);
-        xf::k_fwd_row<LOGN, SINGLE><<<njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(jobs, o);
+        return gfx::chain_launch(xf::k_fwd_row<LOGN, SINGLE>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
+                                 jobs, o);
     } else {
         xf::k_inv_row<LOGN, SINGLE><<<njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(jobs, o);
-        xf::k_inv_col<LOGN, SINGLE><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs, o);
+        return gfx::chain_launch(xf::k_inv_col<LOGN, SINGLE>, true, njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s,
+                                 jobs, o);
     }
-    return cudaGetLastError();
 }
 
 template <int LOGN>
@@ -34,8 +35,8 @@ cudaError_t launch_lift(const xf::Job* jobs, int njobs, cudaStream_t s) {
         cudaFuncSetAttribute(xf::k_fwd_row<LOGN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
     });
     xf::k_fwd_col_lift<LOGN><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs);
-    xf::k_fwd_row<LOGN, false><<<njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(jobs, xf::Job{});
-    return cudaGetLastError();
+    return gfx::chain_launch(xf::k_fwd_row<LOGN, false>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
+                             jobs, xf::Job{});
 }
 
 }  // namespace

@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "ntt.cuh"
+#include "pdl.cuh"
 
 namespace xf {
 
@@ -75,6 +76,7 @@ __device__ __forceinline__ Job get_job(const Job* __restrict__ arr, const Job& o
 template <int LOGN, bool SINGLE>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 k_fwd_col(const Job* __restrict__ arr, const Job one) {
+    gfx::chain_begin();
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::COL_TILES;
@@ -95,6 +97,7 @@ k_fwd_col(const Job* __restrict__ arr, const Job one) {
 template <int LOGN>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 k_fwd_col_lift(const Job* __restrict__ arr) {
+    gfx::chain_begin();
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::COL_TILES;
@@ -113,6 +116,7 @@ k_fwd_col_lift(const Job* __restrict__ arr) {
 template <int LOGN, bool SINGLE>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 k_fwd_row(const Job* __restrict__ arr, const Job one) {
+    gfx::chain_begin();
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::ROW_TILES;
@@ -131,6 +135,7 @@ k_fwd_row(const Job* __restrict__ arr, const Job one) {
 template <int LOGN, bool SINGLE>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::ROW_THREADS, ntt::Geo<LOGN>::ROW_MINB)
 k_inv_row(const Job* __restrict__ arr, const Job one) {
+    gfx::chain_begin();
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::ROW_TILES;
@@ -149,6 +154,7 @@ k_inv_row(const Job* __restrict__ arr, const Job one) {
 template <int LOGN, bool SINGLE>
 __global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
 k_inv_col(const Job* __restrict__ arr, const Job one) {
+    gfx::chain_begin();
     using G = ntt::Geo<LOGN>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::COL_TILES;
