@@ -356,16 +356,20 @@ struct IntAr {
     __device__ __forceinline__ void inv(u64 (&v)[1 << K], const TW& tw, u32 B) const { gs_reg<K>(v, tw, B, q, two_q); }
 };
 
-// Geometry of the two passes for one LOGN.
-template <int LOGN>
+// Geometry of the two passes for one LOGN. W: columns of the column pass's
+// tile at 256 rows, COL_WIDE or COL_NARROW (half the threads per CTA and twice
+// the CTAs, for grids that leave SMs idle; see narrow_tiles).
+constexpr int COL_WIDE = 16, COL_NARROW = 8;
+template <int LOGN, int W = COL_WIDE>
 struct Geo {
     static_assert(LOGN >= 9 && LOGN <= 16, "LOGN out of range");
     static constexpr int N = 1 << LOGN;
     static constexpr int A = LOGN - 8;               // column stages
     static constexpr int R1 = 1 << A;                // rows
     static constexpr int COLS = 256;
-    // column pass: all rows x C columns, <= 4096 elements, >= 16 columns
-    static constexpr int C = cmin(256, cmax(16, 4096 >> A));
+    // column pass: all rows x C columns, <= 256 W elements, >= W columns
+    static constexpr int C = cmin(256, cmax(W, (256 * W) >> A));
+    static constexpr int COL_MINB = 64 / W;
     static constexpr int COL_TILE = R1 * C;
     static constexpr int COL_TILES = COLS / C;
     static constexpr int COL_THREADS = COL_TILE / 16;
@@ -383,6 +387,16 @@ struct Geo {
     static constexpr int COL_SMEM = COL_TILE * 8;
     static constexpr int ROW_SMEM = RB * ROW_STRIDE * 8;
 };
+
+// Column tiles of eight columns where sixteen would fill at most two CTAs of
+// each SM's four: one product (N = 2^15, 16-64 wide tiles a kernel) 89 -> 83 us,
+// a transform of 3 + 3 rotations (N = 2^13, 24-726) 365 -> 356 us. On grids of
+// many waves their 64-byte row segments cost more than they spread: 128 products
+// 6.84 -> 7.03 ms with narrow tiles throughout.
+template <int LOGN>
+inline bool narrow_tiles(unsigned jobs, int sms) {
+    return jobs * (unsigned)Geo<LOGN>::COL_TILES <= 8u * (unsigned)sms;
+}
 
 __device__ __forceinline__ int rowpad(int c) { return c + (c >> 4); }
 

@@ -24,16 +24,22 @@ int sm_count() { return gfx::current_sm_count(); }
 // segment (both kinds interleaved, one launch).
 template <int LOGN, int PATH>
 struct Variant {
+    template <int W>
+    static void col_attrs() {
+        constexpr int SMEM = ntt::Geo<LOGN, W>::COL_SMEM;
+        cudaFuncSetAttribute(p2_inv_col<LOGN, PATH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaFuncSetAttribute(p3_modup_fwd_col<LOGN, PATH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaFuncSetAttribute(p7a_moddown_inv_col<LOGN, PATH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaFuncSetAttribute(p7b_moddown_inv_col<LOGN, PATH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        cudaFuncSetAttribute(p8_moddown_fwd_col<LOGN, PATH, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    }
     static void attrs() {
         using G = ntt::Geo<LOGN>;
+        col_attrs<ntt::COL_WIDE>();
+        col_attrs<ntt::COL_NARROW>();
         cudaFuncSetAttribute(p1_inv_row<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
-        cudaFuncSetAttribute(p2_inv_col<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
-        cudaFuncSetAttribute(p3_modup_fwd_col<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
         cudaFuncSetAttribute(p4_modup_fwd_row<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
         cudaFuncSetAttribute(p6_moddown_inv_row<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
-        cudaFuncSetAttribute(p7a_moddown_inv_col<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
-        cudaFuncSetAttribute(p7b_moddown_inv_col<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
-        cudaFuncSetAttribute(p8_moddown_fwd_col<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
         cudaFuncSetAttribute(p9_final_fwd_row<LOGN, PATH>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
     }
     // Phase k of the jobs in segment PATH (P5 and P7 have one integer kernel
@@ -49,15 +55,22 @@ struct Variant {
             gfx::chain_launch(kernel, after, grid, block, smem, s, D, pd, J);
             after = true;
         };
+        // a column kernel on wide tiles, or on narrow ones where those leave SMs idle
+        const bool narrow = ntt::narrow_tiles<LOGN>(cnt, sm_count());
+        auto run_col = [&](auto* wide, auto* slim) {
+            using N = ntt::Geo<LOGN, ntt::COL_NARROW>;
+            if (narrow) run(slim, cnt * N::COL_TILES, N::COL_THREADS, N::COL_SMEM);
+            else run(wide, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM);
+        };
         switch (k) {
             case 0: run(p1_inv_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
-            case 1: run(p2_inv_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
-            case 2: run(p3_modup_fwd_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case 1: run_col(p2_inv_col<LOGN, PATH, ntt::COL_WIDE>, p2_inv_col<LOGN, PATH, ntt::COL_NARROW>); break;
+            case 2: run_col(p3_modup_fwd_col<LOGN, PATH, ntt::COL_WIDE>, p3_modup_fwd_col<LOGN, PATH, ntt::COL_NARROW>); break;
             case 3: run(p4_modup_fwd_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
             case 5: run(p6_moddown_inv_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
-            case 6: run(p7a_moddown_inv_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
-            case NPHASE: run(p7b_moddown_inv_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
-            case 7: run(p8_moddown_fwd_col<LOGN, PATH>, cnt * G::COL_TILES, G::COL_THREADS, G::COL_SMEM); break;
+            case 6: run_col(p7a_moddown_inv_col<LOGN, PATH, ntt::COL_WIDE>, p7a_moddown_inv_col<LOGN, PATH, ntt::COL_NARROW>); break;
+            case NPHASE: run_col(p7b_moddown_inv_col<LOGN, PATH, ntt::COL_WIDE>, p7b_moddown_inv_col<LOGN, PATH, ntt::COL_NARROW>); break;
+            case 7: run_col(p8_moddown_fwd_col<LOGN, PATH, ntt::COL_WIDE>, p8_moddown_fwd_col<LOGN, PATH, ntt::COL_NARROW>); break;
             case 8: run(p9_final_fwd_row<LOGN, PATH>, cnt * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM); break;
             default: break;
         }

@@ -157,9 +157,9 @@ __device__ __forceinline__ void on_path(uint2& jb, F&& f) {
 constexpr int CS_VB = 2;
 constexpr int P8_VB = 1;   // P8 carries more live state per pair (three modes inlined)
 
-template <int LOGN>
+template <int LOGN, int W>
 struct ColStage {
-    using G = ntt::Geo<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
     static constexpr int VPR = G::C / 2;
     static constexpr int PER = G::R1 * VPR / G::COL_THREADS;
     static_assert(PER * G::COL_THREADS == G::R1 * VPR && PER % CS_VB == 0, "column staging geometry");
@@ -348,10 +348,10 @@ p1_inv_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __re
 }
 
 // ------------------------------------------------------------------ P2
-template <int LOGN, bool FP>
+template <int LOGN, int W, bool FP>
 __device__ __forceinline__ void p2_inv_col_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
                                               const u32 tile) {
-    using G = ntt::Geo<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     const int c0 = tile * G::C;
     const PairDesc& P = pairs[jb.x];
@@ -376,21 +376,21 @@ __device__ __forceinline__ void p2_inv_col_body(const DevCtx& D, const PairDesc*
     }
 }
 
-template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, int PATH, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 p2_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     gfx::chain_begin();
-    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
-    const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
-    on_path<PATH>(jb, [&](auto fp) { p2_inv_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
+    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN, W>::COL_TILES];
+    const u32 tile = blockIdx.x % ntt::Geo<LOGN, W>::COL_TILES;
+    on_path<PATH>(jb, [&](auto fp) { p2_inv_col_body<LOGN, W, decltype(fp)::value>(D, pairs, jb, tile); });
 }
 
 // ------------------------------------------------------------------ P3
-template <int LOGN, bool FP>
+template <int LOGN, int W, bool FP>
 __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
                                               const u32 tile) {
-    using G = ntt::Geo<LOGN>;
-    using CS = ColStage<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
+    using CS = ColStage<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     __shared__ ConvTerm cst[MAXA];
     const int c0 = tile * G::C;
@@ -483,13 +483,13 @@ __device__ __forceinline__ void p3_modup_fwd_col_body(const DevCtx& D, const Pai
     ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P3_IN>(sm, twf_of<FP>(D, qp, LOGN), ar, ld, stf);
 }
 
-template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, int PATH, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 p3_modup_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     gfx::chain_begin();
-    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
-    const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
-    on_path<PATH>(jb, [&](auto fp) { p3_modup_fwd_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
+    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN, W>::COL_TILES];
+    const u32 tile = blockIdx.x % ntt::Geo<LOGN, W>::COL_TILES;
+    on_path<PATH>(jb, [&](auto fp) { p3_modup_fwd_col_body<LOGN, W, decltype(fp)::value>(D, pairs, jb, tile); });
 }
 
 // P3, warp-specialised form: a persistent CTA of COL_THREADS transform threads
@@ -1708,10 +1708,10 @@ p6_moddown_inv_row(const DevCtx D, const PairDesc* __restrict__ pairs, const uin
 // Key), then r_l = u - conv'_l * P^-1 mod q_l into U[c], with the P->q_l
 // constants folding P^-1 (and 2^64 for a Montgomery reduction when
 // D.mont_down). Both read P6's output in the path's own word format.
-template <int LOGN, bool FP>
+template <int LOGN, int W, bool FP>
 __device__ __forceinline__ void p7a_moddown_inv_col_body(const DevCtx& D, const PairDesc* __restrict__ pairs,
                                                          const uint2 jb, const u32 tile) {
-    using G = ntt::Geo<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     const int c0 = tile * G::C;
     const PairDesc& P = pairs[jb.x];
@@ -1736,20 +1736,20 @@ __device__ __forceinline__ void p7a_moddown_inv_col_body(const DevCtx& D, const 
     }
 }
 
-template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, int PATH, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 p7a_moddown_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     gfx::chain_begin();
-    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
-    const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
-    on_path<PATH>(jb, [&](auto fp) { p7a_moddown_inv_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
+    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN, W>::COL_TILES];
+    const u32 tile = blockIdx.x % ntt::Geo<LOGN, W>::COL_TILES;
+    on_path<PATH>(jb, [&](auto fp) { p7a_moddown_inv_col_body<LOGN, W, decltype(fp)::value>(D, pairs, jb, tile); });
 }
 
-template <int LOGN, bool FP>
+template <int LOGN, int W, bool FP>
 __device__ __forceinline__ void p7b_moddown_inv_col_body(const DevCtx& D, const PairDesc* __restrict__ pairs,
                                                          const uint2 jb, const u32 tile) {
-    using G = ntt::Geo<LOGN>;
-    using CS = ColStage<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
+    using CS = ColStage<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     __shared__ ConvTerm cl_[gfx::MAXP];
     const int c0 = tile * G::C;
@@ -1811,21 +1811,21 @@ __device__ __forceinline__ void p7b_moddown_inv_col_body(const DevCtx& D, const 
     }
 }
 
-template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, int PATH, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 p7b_moddown_inv_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     gfx::chain_begin();
-    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
-    const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
-    on_path<PATH>(jb, [&](auto fp) { p7b_moddown_inv_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
+    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN, W>::COL_TILES];
+    const u32 tile = blockIdx.x % ntt::Geo<LOGN, W>::COL_TILES;
+    on_path<PATH>(jb, [&](auto fp) { p7b_moddown_inv_col_body<LOGN, W, decltype(fp)::value>(D, pairs, jb, tile); });
 }
 
 // ------------------------------------------------------------------ P8
-template <int LOGN, u32 MODE, bool FP>
+template <int LOGN, int W, u32 MODE, bool FP>
 __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 c, u32 i, int c0, u64* sm,
                                         const ConvTerm* ci) {
-    using G = ntt::Geo<LOGN>;
-    using CS = ColStage<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
+    using CS = ColStage<LOGN, W>;
     const u32 L = P.L, K = D.K, l = L - 1;
     const WsLayout w = ws_layout(L, K, D.alpha);
     const Level& lv = D.lvl[L];
@@ -1933,12 +1933,12 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
     ntt::fwd_col_rounds<G::A, G::C, G::COL_THREADS, 0, P8_IN>(sm, twf_of<FP>(D, i, LOGN), ar, ld, st);
 }
 
-template <int LOGN, bool FP>
+template <int LOGN, int W, bool FP>
 __device__ __forceinline__ void p8_moddown_fwd_col_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
                                               const u32 tile) {
     extern __shared__ __align__(16) u64 sm[];
     __shared__ ConvTerm ci[gfx::MAXP + 1];
-    const int c0 = tile * ntt::Geo<LOGN>::C;
+    const int c0 = tile * ntt::Geo<LOGN, W>::C;
     const PairDesc& P = pairs[jb.x];
     const u32 c = jb.y / P.L, i = jb.y % P.L;
     const bool quot = FP && D.wrap_down;
@@ -1959,18 +1959,18 @@ __device__ __forceinline__ void p8_moddown_fwd_col_body(const DevCtx& D, const P
         ci[D.K] = conv_term<false>(D.lvl[P.L].s2[i], D.mod[i]);
     }
     __syncthreads();
-    if (P.mode == EMR) p8_body<LOGN, EMR, FP>(D, P, c, i, c0, sm, ci);
-    else if (P.mode == RESCALE) p8_body<LOGN, RESCALE, FP>(D, P, c, i, c0, sm, ci);
-    else p8_body<LOGN, KS, FP>(D, P, c, i, c0, sm, ci);
+    if (P.mode == EMR) p8_body<LOGN, W, EMR, FP>(D, P, c, i, c0, sm, ci);
+    else if (P.mode == RESCALE) p8_body<LOGN, W, RESCALE, FP>(D, P, c, i, c0, sm, ci);
+    else p8_body<LOGN, W, KS, FP>(D, P, c, i, c0, sm, ci);
 }
 
-template <int LOGN, int PATH>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, int PATH, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 p8_moddown_fwd_col(const DevCtx D, const PairDesc* __restrict__ pairs, const uint2* __restrict__ jobs) {
     gfx::chain_begin();
-    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN>::COL_TILES];
-    const u32 tile = blockIdx.x % ntt::Geo<LOGN>::COL_TILES;
-    on_path<PATH>(jb, [&](auto fp) { p8_moddown_fwd_col_body<LOGN, decltype(fp)::value>(D, pairs, jb, tile); });
+    uint2 jb = jobs[blockIdx.x / ntt::Geo<LOGN, W>::COL_TILES];
+    const u32 tile = blockIdx.x % ntt::Geo<LOGN, W>::COL_TILES;
+    on_path<PATH>(jb, [&](auto fp) { p8_moddown_fwd_col_body<LOGN, W, decltype(fp)::value>(D, pairs, jb, tile); });
 }
 
 // ------------------------------------------------------------------ P9

@@ -4,39 +4,52 @@
 
 namespace {
 
-template <int LOGN, bool SINGLE>
-cudaError_t launch_t(const xf::Job* jobs, const xf::Job* one, int njobs, bool inverse, cudaStream_t s) {
-    using G = ntt::Geo<LOGN>;
+// One transform with column tiles of W columns (ntt::narrow_tiles).
+template <int LOGN, bool SINGLE, int W>
+cudaError_t launch_w(const xf::Job* jobs, const xf::Job& o, int njobs, bool inverse, cudaStream_t s) {
+    using G = ntt::Geo<LOGN, W>;
     static gfx::DeviceOnce attrs;   // shared-memory limits, once per device
     attrs([] {
-        cudaFuncSetAttribute(xf::k_fwd_col<LOGN, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
-        cudaFuncSetAttribute(xf::k_inv_col<LOGN, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
+        cudaFuncSetAttribute(xf::k_fwd_col<LOGN, SINGLE, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
+        cudaFuncSetAttribute(xf::k_inv_col<LOGN, SINGLE, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
         cudaFuncSetAttribute(xf::k_fwd_row<LOGN, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
         cudaFuncSetAttribute(xf::k_inv_row<LOGN, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
     });
-    const xf::Job o = one ? *one : xf::Job{};
     if (!inverse) {
-        xf::k_fwd_col<LOGN, SINGLE><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs, o);
+        xf::k_fwd_col<LOGN, SINGLE, W><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs, o);
         return gfx::chain_launch(xf::k_fwd_row<LOGN, SINGLE>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
                                  jobs, o);
-    } else {
-        xf::k_inv_row<LOGN, SINGLE><<<njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(jobs, o);
-        return gfx::chain_launch(xf::k_inv_col<LOGN, SINGLE>, true, njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s,
-                                 jobs, o);
     }
+    xf::k_inv_row<LOGN, SINGLE><<<njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(jobs, o);
+    return gfx::chain_launch(xf::k_inv_col<LOGN, SINGLE, W>, true, njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s,
+                             jobs, o);
+}
+
+template <int LOGN, bool SINGLE>
+cudaError_t launch_t(const xf::Job* jobs, const xf::Job* one, int njobs, bool inverse, cudaStream_t s) {
+    const xf::Job o = one ? *one : xf::Job{};
+    return ntt::narrow_tiles<LOGN>(njobs, gfx::current_sm_count())
+               ? launch_w<LOGN, SINGLE, ntt::COL_NARROW>(jobs, o, njobs, inverse, s)
+               : launch_w<LOGN, SINGLE, ntt::COL_WIDE>(jobs, o, njobs, inverse, s);
+}
+
+template <int LOGN, int W>
+cudaError_t launch_lift_w(const xf::Job* jobs, int njobs, cudaStream_t s) {
+    using G = ntt::Geo<LOGN, W>;
+    static gfx::DeviceOnce attrs;
+    attrs([] {
+        cudaFuncSetAttribute(xf::k_fwd_col_lift<LOGN, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
+        cudaFuncSetAttribute(xf::k_fwd_row<LOGN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
+    });
+    xf::k_fwd_col_lift<LOGN, W><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs);
+    return gfx::chain_launch(xf::k_fwd_row<LOGN, false>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
+                             jobs, xf::Job{});
 }
 
 template <int LOGN>
 cudaError_t launch_lift(const xf::Job* jobs, int njobs, cudaStream_t s) {
-    using G = ntt::Geo<LOGN>;
-    static gfx::DeviceOnce attrs;
-    attrs([] {
-        cudaFuncSetAttribute(xf::k_fwd_col_lift<LOGN>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
-        cudaFuncSetAttribute(xf::k_fwd_row<LOGN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
-    });
-    xf::k_fwd_col_lift<LOGN><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs);
-    return gfx::chain_launch(xf::k_fwd_row<LOGN, false>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
-                             jobs, xf::Job{});
+    return ntt::narrow_tiles<LOGN>(njobs, gfx::current_sm_count()) ? launch_lift_w<LOGN, ntt::COL_NARROW>(jobs, njobs, s)
+                                                                   : launch_lift_w<LOGN, ntt::COL_WIDE>(jobs, njobs, s);
 }
 
 }  // namespace

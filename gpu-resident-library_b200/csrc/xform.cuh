@@ -73,11 +73,11 @@ __device__ __forceinline__ Job get_job(const Job* __restrict__ arr, const Job& o
     else return arr[i];
 }
 
-template <int LOGN, bool SINGLE>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, bool SINGLE, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 k_fwd_col(const Job* __restrict__ arr, const Job one) {
     gfx::chain_begin();
-    using G = ntt::Geo<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::COL_TILES;
     const int c0 = (blockIdx.x % G::COL_TILES) * G::C;
@@ -94,11 +94,11 @@ k_fwd_col(const Job* __restrict__ arr, const Job one) {
 // in coefficient form, centred mod q0, into every tower; plaintext embedding:
 // signed 64-bit coefficients into every tower), written to job.x: the lift
 // and the first transform pass in one read of the source.
-template <int LOGN>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 k_fwd_col_lift(const Job* __restrict__ arr) {
     gfx::chain_begin();
-    using G = ntt::Geo<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::COL_TILES;
     const int c0 = (blockIdx.x % G::COL_TILES) * G::C;
@@ -151,11 +151,11 @@ k_inv_row(const Job* __restrict__ arr, const Job one) {
     });
 }
 
-template <int LOGN, bool SINGLE>
-__global__ void __launch_bounds__(ntt::Geo<LOGN>::COL_THREADS, 4)
+template <int LOGN, bool SINGLE, int W>
+__global__ void __launch_bounds__(ntt::Geo<LOGN, W>::COL_THREADS, ntt::Geo<LOGN, W>::COL_MINB)
 k_inv_col(const Job* __restrict__ arr, const Job one) {
     gfx::chain_begin();
-    using G = ntt::Geo<LOGN>;
+    using G = ntt::Geo<LOGN, W>;
     extern __shared__ __align__(16) u64 sm[];
     const int job = blockIdx.x / G::COL_TILES;
     const int c0 = (blockIdx.x % G::COL_TILES) * G::C;

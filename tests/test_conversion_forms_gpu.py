@@ -32,6 +32,7 @@ def residues(rng, mods, n, edge):
     (1024, (60, 30, 40, 30, 45, 49), 2, 3, 60),      # narrow towers
     (1024, (60, 55, 55, 50, 55), 2, 2, 60),
     (4096, (50, 60, 50, 60, 50), 4, 4, 55),
+    (1024, (61, 61, 50, 61), 2, 2, 61),              # the widest towers: 8q just below 2^64
 ])
 def test_conversion_forms(n, bits, K, alpha, pbits):
     import gpufhe_b200 as G
