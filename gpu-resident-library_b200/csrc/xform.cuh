@@ -60,9 +60,8 @@ __device__ __forceinline__ void with_path(const Job& j, F&& f) {
         else f(ntt::FpAr{qd, qi, j.q}, ntt::TwDConv{j.w});
         return;
     }
-    const ntt::IntAr ar{j.q, 2 * j.q};
-    if (j.tw) f(ar, ntt::TwPacked{j.tw});
-    else f(ar, ntt::TwSplit{j.w, j.wp});
+    if (j.tw) f(ntt::IntAr{j.q, 2 * j.q}, ntt::TwPacked{j.tw});
+    else f(ntt::IntArWide{j.q, 2 * j.q}, ntt::TwSplit{j.w, j.wp});
 }
 
 // Jobs come either from a device array (SINGLE = false) or a single by-value
