@@ -459,8 +459,8 @@ struct Geo {
     static constexpr int ROW_SMEM = RB * ROW_STRIDE * 8;
 };
 
-// Column tiles of eight columns where sixteen would fill at most two CTAs of
-// each SM's four: one product (N = 2^15, 16-64 wide tiles a kernel) 89 -> 83 us,
+// Column tiles of eight columns where sixteen would make at most two waves (of
+// four CTAs per SM): one product (N = 2^15, 16-64 wide tiles a kernel) 89 -> 83 us,
 // a transform of 3 + 3 rotations (N = 2^13, 24-726) 365 -> 356 us. On grids of
 // many waves their 64-byte row segments cost more than they spread: 128 products
 // 6.84 -> 7.03 ms with narrow tiles throughout.

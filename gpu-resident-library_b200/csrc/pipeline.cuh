@@ -100,6 +100,16 @@ __device__ __forceinline__ u32 galois_slot(u32 j, u64 k) {
     return __brev((t - 1) >> 1) >> (32 - LOGN);
 }
 
+// The slots of an aligned block of 2^m come from one aligned block of 2^m
+// (the low bits of brv(j) k depend only on the low bits of brv(j), which are
+// j's high ones), permuted inside it. So a rotated tile is read as whole rows
+// and permuted in shared memory: word by word from global memory a warp
+// touched up to 32 sectors per load where a row segment has eight.
+template <int LOGN, int BLOCK>
+__device__ __forceinline__ u32 galois_block(u32 j, u64 k) {
+    return galois_slot<LOGN>(j, k) & ~(u32)(BLOCK - 1);
+}
+
 // Digit source value at element e of Q tower i (eval form, canonical).
 template <int LOGN>
 __device__ __forceinline__ u64 digit_src(const PairDesc& P, u32 i, u32 e, const ModC& m) {
@@ -1215,8 +1225,11 @@ p5_mac_async(const DevCtx D, const PairDesc* __restrict__ pairs, const uint4* __
 // count. P5T_NC consumer threads own one 16-byte pair of the tile each,
 // release a stage by arriving on its empty mbarrier as soon as they hold its
 // words in registers, and then write the epilogue. The key tile of row r
-// arrives the same way, once per CTA. Hoisted-rotation digits (an eval-slot
-// gather) and the rotation source are read by the consumers directly.
+// arrives the same way, once per CTA. Rotated rows (the rotation source, a
+// hoisted rotation's digits) arrive as their source block, which the consumers
+// read permuted (gathered from global memory by the consumers, the same forms
+// took 841 instead of 649 us for 48 hoisted rotations at N = 2^16, 735 instead
+// of 659 for plain ones).
 // Every wait is bounded in time (mbar_wait): when one expires the thread ORs
 // a code into D.err and leaves, and the producer waits (bounded again) for
 // its copies in flight to land before it leaves, so no copy outlives the CTA.
@@ -1316,9 +1329,9 @@ __device__ __forceinline__ bool p5t_setup(const DevCtx& D, u64* sm, P5Ring<S>& R
 }
 
 // The producer (one thread): the key tile of row r once, then per listed
-// pair the tensor inputs (EvalMult+Rescale, slots 0-3) or the keyswitch input
-// (slot 1) of a Q row and every other digit of its tower (slot MACA_IN + p),
-// into stage g % S after the consumers have released it; finally it waits
+// pair the tensor inputs (EvalMult+Rescale, slots 0-3) or the keyswitch or
+// rotation source (slot 1) of a Q row and every other digit of its tower (slot
+// MACA_IN + p; rotated ones as their source block), into stage g % S after the consumers have released it; finally it waits
 // (bounded) for every copy in flight.
 template <int LOGN, int S>
 __device__ __forceinline__ void p5t_produce(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint4 jb,
@@ -1346,20 +1359,23 @@ __device__ __forceinline__ void p5t_produce(const DevCtx& D, const PairDesc* __r
         const u32 pin = is_p ? 0xffffffffu : i / D.alpha;
         const WsLayout w = ws_layout(L, K, D.alpha);
         const u32 nparts = D.lvl[L].nparts;
-        const u32 nin = is_p ? 0u : (P.mode == EMR ? 4u : (P.mode == KS ? 1u : 0u));
-        const u32 ndig = P.mode == HROT ? 0u : nparts - (pin < nparts ? 1u : 0u);
+        const u32 nin = is_p ? 0u : (P.mode == EMR ? 4u : 1u);
+        const u32 ndig = nparts - (pin < nparts ? 1u : 0u);
         u64* sb = R.stage + (size_t)b * slots * P5T_TILE;
-        const size_t o = ((size_t)i << LOGN) + tile0;
+        const bool rot = P.mode == ROT || P.mode == HROT;
+        const u32 src0 = rot ? galois_block<LOGN, P5T_TILE>(tile0, P.galois) : tile0;
+        const size_t o = ((size_t)i << LOGN) + src0;
         mbar_arrive_expect_tx(R.full(b), (nin + ndig) * ROW);
         if (nin == 4) {
             for (u32 k = 0; k < 4; ++k) bulk_load(smem_addr(sb + k * P5T_TILE), P.in[k] + o, ROW, R.full(b));
         } else if (nin == 1) {
-            bulk_load(smem_addr(sb + P5T_TILE), P.in[0] + o, ROW, R.full(b));
+            bulk_load(smem_addr(sb + P5T_TILE), P.in[rot ? 1 : 0] + o, ROW, R.full(b));
         }
+        const u32 dig0 = P.mode == HROT ? src0 : tile0;
         if (ndig)
             for (u32 p = 0; p < nparts; ++p) {
                 if (p == pin) continue;
-                const u64* Yt = P.ysrc + ((size_t)(w.Y + p * QlP + i) << LOGN) + tile0;
+                const u64* Yt = P.ysrc + ((size_t)(w.Y + p * QlP + i) << LOGN) + dig0;
                 bulk_load(smem_addr(sb + R.slot(p, pin) * P5T_TILE), Yt, ROW, R.full(b));
             }
         issued = g + 1;
@@ -1399,12 +1415,18 @@ __device__ __forceinline__ void p5t_consume_int(const DevCtx& D, const PairDesc*
         const u32 nparts = lv.nparts;
         const u32 pin = is_p ? 0xffffffffu : i / D.alpha;
         const bool emr = P.mode == EMR;
-        const u64* sb = R.stage + (size_t)b * slots * P5T_TILE + e;
+        const u64* sb = R.stage + (size_t)b * slots * P5T_TILE;
+        const bool rot = P.mode == ROT || P.mode == HROT;
+        u32 g0 = 0, g1 = 0;                     // this thread's words in a rotated row's source block
+        if (rot) {
+            g0 = galois_slot<LOGN>(tile0 + e, P.galois) & (P5T_TILE - 1);
+            g1 = galois_slot<LOGN>(tile0 + e + 1, P.galois) & (P5T_TILE - 1);
+        }
         ulonglong2 s{0, 0}, t0{0, 0}, t1{0, 0};
         if (!is_p) {
             if (emr) {
-                const ulonglong2 x0 = ld2(sb), x1 = ld2(sb + P5T_TILE);
-                const ulonglong2 y0 = ld2(sb + 2 * P5T_TILE), y1 = ld2(sb + 3 * P5T_TILE);
+                const ulonglong2 x0 = ld2(sb + e), x1 = ld2(sb + P5T_TILE + e);
+                const ulonglong2 y0 = ld2(sb + 2 * P5T_TILE + e), y1 = ld2(sb + 3 * P5T_TILE + e);
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     const u64 a0 = v2get(x0, j), a1 = v2get(x1, j), b0 = v2get(y0, j), b1 = v2get(y1, j);
@@ -1418,13 +1440,8 @@ __device__ __forceinline__ void p5t_consume_int(const DevCtx& D, const PairDesc*
                     v2set(t1, j, acc_reduce(lo, hi, m, D.mont));
                 }
             } else {
-                if (P.mode == ROT || P.mode == HROT) {
-                    const u64* src = P.in[1] + ((size_t)i << LOGN);
-#pragma unroll
-                    for (int j = 0; j < 2; ++j) v2set(s, j, src[galois_slot<LOGN>(tile0 + e + j, P.galois)]);
-                } else {
-                    s = ld2(sb + P5T_TILE);
-                }
+                if (rot) s = make_ulonglong2(sb[P5T_TILE + g0], sb[P5T_TILE + g1]);
+                else s = ld2(sb + P5T_TILE + e);
                 if (D.mont) {
 #pragma unroll
                     for (int j = 0; j < 2; ++j) v2set(s, j, redc(v2get(s, j), 0, m));
@@ -1436,12 +1453,10 @@ __device__ __forceinline__ void p5t_consume_int(const DevCtx& D, const PairDesc*
             ulonglong2 dv;
             if (p == pin) {
                 dv = s;
-            } else if (P.mode == HROT) {            // sigma_k of the shared digit: eval-slot gather
-                const u64* Yt = P.ysrc + ((size_t)(w.Y + p * QlP + i) << LOGN);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) v2set(dv, j, Yt[galois_slot<LOGN>(tile0 + e + j, P.galois)]);
             } else {
-                dv = ld2(sb + R.slot(p, pin) * P5T_TILE);
+                const u64* dg = sb + R.slot(p, pin) * P5T_TILE;
+                if (P.mode == HROT) dv = make_ulonglong2(dg[g0], dg[g1]);   // sigma_k of the shared digit
+                else dv = ld2(dg + e);
             }
             const ulonglong2 kbv = ld2(R.keys + (2 * p) * P5T_TILE + e);
             const ulonglong2 kav = ld2(R.keys + (2 * p + 1) * P5T_TILE + e);
@@ -1558,11 +1573,12 @@ __device__ __forceinline__ void p5t_consume_fp(const DevCtx& D, const PairDesc* 
         const WsLayout w = ws_layout(L, K, D.alpha);
         const u32 nparts = lv.nparts;
         const bool emr = P.mode == EMR;
-        const u64* sb = R.stage + (size_t)b * slots * P5T_TILE + e;
+        const u64* sb = R.stage + (size_t)b * slots * P5T_TILE;
+        u32 g0 = 0, g1 = 0;                     // this thread's words in a rotated row's source block
         double s[2], t0[2] = {0.0, 0.0}, t1[2] = {0.0, 0.0};
         if (emr) {
-            const ulonglong2 x0 = ld2(sb), x1 = ld2(sb + P5T_TILE);
-            const ulonglong2 y0 = ld2(sb + 2 * P5T_TILE), y1 = ld2(sb + 3 * P5T_TILE);
+            const ulonglong2 x0 = ld2(sb + e), x1 = ld2(sb + P5T_TILE + e);
+            const ulonglong2 y0 = ld2(sb + 2 * P5T_TILE + e), y1 = ld2(sb + 3 * P5T_TILE + e);
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const double a0 = ntt::u2d(v2get(x0, j)), a1 = ntt::u2d(v2get(x1, j));
@@ -1572,11 +1588,12 @@ __device__ __forceinline__ void p5t_consume_fp(const DevCtx& D, const PairDesc* 
                 t1[j] = __dadd_rn(ar.mulq<false>(a0, b1), ar.mulq<false>(a1, b0));
             }
         } else if (P.mode == ROT || P.mode == HROT) {
-            const u64* src = P.in[1] + ((size_t)i << LOGN);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) s[j] = ntt::u2d(src[galois_slot<LOGN>(tile0 + e + j, P.galois)]);
+            g0 = galois_slot<LOGN>(tile0 + e, P.galois) & (P5T_TILE - 1);
+            g1 = galois_slot<LOGN>(tile0 + e + 1, P.galois) & (P5T_TILE - 1);
+            s[0] = ntt::u2d(sb[P5T_TILE + g0]);
+            s[1] = ntt::u2d(sb[P5T_TILE + g1]);
         } else {
-            const ulonglong2 x = ld2(sb + P5T_TILE);
+            const ulonglong2 x = ld2(sb + P5T_TILE + e);
             s[0] = ntt::u2d(x.x);
             s[1] = ntt::u2d(x.y);
         }
@@ -1586,12 +1603,11 @@ __device__ __forceinline__ void p5t_consume_fp(const DevCtx& D, const PairDesc* 
             if (p == pin) {
                 y[0] = s[0];
                 y[1] = s[1];
-            } else if (P.mode == HROT) {        // sigma_k of the shared digit: eval-slot gather
-                const u64* Yt = P.ysrc + ((size_t)(w.Y + p * QlP + i) << LOGN);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) y[j] = ntt::u2d(Yt[galois_slot<LOGN>(tile0 + e + j, P.galois)]);
             } else {
-                const ulonglong2 dv = ld2(sb + R.slot(p, pin) * P5T_TILE);
+                const u64* dg = sb + R.slot(p, pin) * P5T_TILE;
+                ulonglong2 dv;
+                if (P.mode == HROT) dv = make_ulonglong2(dg[g0], dg[g1]);   // sigma_k of the shared digit
+                else dv = ld2(dg + e);
                 y[0] = ntt::u2d(dv.x);
                 y[1] = ntt::u2d(dv.y);
             }
@@ -1996,21 +2012,47 @@ __device__ __forceinline__ void p9_final_fwd_row_body(const DevCtx& D, const Pai
     const u64* Wt = slot_ptr(P, w.W + c * L + i, LOGN) + tile0;
     const Level& lv = D.lvl[L];
     const u64 s1 = lv.s1[i], s1p = lv.s1p[i];
+    // A rotation's c0 under sigma_k: each warp reads its rows' source blocks whole,
+    // parks one row at a time in the row's shared memory once the transform's words
+    // are in registers, and reads it permuted: P9 of 48 rotations 392 -> 303 us
+    // against gathering c0 word by word.
+    if (c == 0 && (mode == ROT || mode == HROT)) {
+        const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const u64* c0s = P.in[0] + ((size_t)i << LOGN);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            const u32 row0 = (u32)tile0 + (wl * 2 + h) * 256;      // tower index of this row's first slot
+            const u64* src = c0s + galois_block<LOGN, 256>(row0, P.galois);
+            u64* srow = sm + (wl * 2 + h) * G::ROW_STRIDE;
+            u64 a[8], x[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                a[k] = Wt[(wl * 2 + h) * 256 + lane + 32 * k];
+                x[k] = src[lane + 32 * k];
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                a[k] = csub(a[k] + ar.final_canon(srow[ntt::rowpad(lane) + 34 * k]), m.q);
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) srow[ntt::rowpad(lane) + 34 * k] = x[k];
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int cc = lane + 32 * k;
+                const int g = (int)(galois_slot<LOGN>(row0 + cc, P.galois) & 255u);
+                out[(wl * 2 + h) * 256 + cc] = csub(a[k] + srow[ntt::rowpad(g)], m.q);
+            }
+        }
+        return;
+    }
     // every W (or rescale input) word of the thread is loaded before the sums
     const u64* addend = mode == RESCALE ? P.in[0] + o : Wt;
     ntt::row_tile_stage<G::RB, G::ROW_THREADS>(
         [&](int e) { return addend[e]; },
         [&](int e, int si, u64 a) {
             const u64 v = ar.final_canon(sm[si]);
-            u64 r;
-            if (mode == RESCALE) {
-                r = csub(shoup(a, s1, s1p, m.q) + v, m.q);
-            } else {
-                r = csub(a + v, m.q);
-                if ((mode == ROT || mode == HROT) && c == 0)
-                    r = csub(r + P.in[0][((size_t)i << LOGN) + galois_slot<LOGN>((u32)(tile0 + e), P.galois)], m.q);
-            }
-            out[e] = r;
+            out[e] = csub((mode == RESCALE ? shoup(a, s1, s1p, m.q) : a) + v, m.q);
         });
 }
 
