@@ -249,16 +249,13 @@ __host__ __device__ constexpr int fwd_bound(int A, int x0) {
 // sums n terms with an error of at most 2^(b-54) (n (n+1) / 2 + 5 n / 2); K is
 // S rounded to a multiple of 2^12 (error 2^11). Where conv_wrap_ok admits (n,
 // b), |r1| < 2^13 q < 2^63, and a second step, K2 = r1 / q rounded, leaves
-// |r| <= q/2 + 1, which the transform takes as it is. Measured: P8 of 128
+// |r| <= q/2 + 1, which the transform takes as it is. Words become doubles by
+// the conversion instruction: two FP64 additions of biased halves took four
+// issue slots (P8 of 128 products 960 -> 912 us). Measured before that: P8 of 128
 // products (N = 2^16, four terms) 1078 -> 966 us, of 48 rotations 492 -> 431 us,
 // of 13 mixed operations (N = 2^14, nine terms) 72 -> 65 us. In P3 and P7 the
 // same form gained nothing: their 50-bit sources already go to exact FP64
 // products, and P7's one conversion per component is not what it waits for.
-constexpr double SIGNED_BIAS = 0x1p84 + 0x1p63 + 0x1p52;   // exact (33 bits)
-__device__ __forceinline__ double x2d(u64 x) {   // RN(x), x < 2^63
-    const double h = __hiloint2double(0x45300000, (int)(x >> 32)), l = __hiloint2double(0x43300000, (int)x);
-    return __dadd_rn(__dsub_rn(h, 0x1.00000001p84), l);
-}
 // ConvTerm of the residue c (canonical mod q), negated when NEG.
 template <bool NEG>
 __device__ __forceinline__ ConvTerm conv_term(u64 c, const ModC& m) {
@@ -287,7 +284,7 @@ __device__ __forceinline__ void quot_terms(u64 (&lo)[VB][2], double (&s)[VB][2],
                     for (int j = 0; j < 2; ++j) {
                         const u64 x = j ? xv[tt][b].y : xv[tt][b].x;
                         lo[b][j] += x * c.c;
-                        s[b][j] = __fma_rn(x2d(x), c.f, s[b][j]);
+                        s[b][j] = __fma_rn(__ull2double_rn(x), c.f, s[b][j]);
                     }
             }
     }
@@ -300,9 +297,7 @@ struct WrapConv {
     __device__ __forceinline__ long long finish(u64 lo, double s) const {
         const long long k = __double_as_longlong(__dadd_rn(s, 0x1.8p64)) - 0x43F8000000000000ll;
         const u64 r1 = lo - (u64)k * (q << 12);
-        const double h = __hiloint2double(0x45300000, (int)(r1 >> 32) ^ (int)0x80000000);
-        const double rd = __dadd_rn(__dsub_rn(h, SIGNED_BIAS),
-                                    __hiloint2double(0x43300000, (int)r1));
+        const double rd = __ll2double_rn((long long)r1);
         const int k2 = __double2loint(__fma_rn(rd, qinv, ntt::FP_M1));
         return (long long)(r1 - (u64)(long long)k2 * q);
     }
@@ -1888,7 +1883,7 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
                             const ConvTerm t = ci[K];
                             const u64 x = j ? xr[b].y : xr[b].x;
                             lo[b][j] += x * t.c + (x > half ? 1ull : 0ull);
-                            sq[b][j] = __fma_rn(x2d(x), t.f, sq[b][j]);
+                            sq[b][j] = __fma_rn(__ull2double_rn(x), t.f, sq[b][j]);
                         }
                         v[j] = wc.finish_d(lo[b][j], sq[b][j]);
                     }
