@@ -91,8 +91,8 @@ cudaError_t launch(const Plan& p, cudaStream_t s, unsigned mask = 0x1ff);
 // candidate with CUDA events on `s` (one dimension at a time on the phases it
 // changes; two interleaved passes, best of three launches each; a candidate
 // wins only if 1.5% faster) and caching the winner. Timing re-runs the batch, so it is skipped (defaults
-// kept) when `measure` is false, while `s` is capturing a graph, or when an
-// operation writes over its own input (in-place rescale).
+// kept) when `measure` is false, while `s` is capturing a graph, or when a
+// rescale writes over an input of the batch (its own or another operation's).
 void tune(Plan& p, cudaStream_t s, bool measure = true);
 constexpr int MAC_MAX_DNUM = 16;
 // P5 forms: register prefetch with 128 threads x 4 words, the cp.async
