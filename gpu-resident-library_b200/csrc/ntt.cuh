@@ -15,10 +15,10 @@
 //
 // Two arithmetic policies run the same rounds. IntAr: 64-bit integer
 // Harvey lazy butterflies with Shoup twiddles (forward values in [0,8q),
-// inverse in [0,2q)), q < 2^61 (IntArWide: [0,4q), q < 2^62). FpAr (q < 2^50): residues held as signed
-// FP64 integers and multiplied exactly with FMA (see FpAr), which runs on
-// the FP64 pipe at about twice the integer path's butterfly rate. Both give
-// the same canonical residues, so callers pick per tower.
+// inverse in [0,2q)), q < 2^61 (IntArWide: [0,4q), q < 2^62). FpArS and FpAr
+// (q < 2^50): residues held as signed FP64 integers and multiplied exactly with
+// FMA, which runs on the FP64 pipe at about twice the integer path's butterfly
+// rate. Both give the same canonical residues, so callers pick per tower.
 //
 // Twiddle index of line-local stage j: a round that starts at stage J0 with
 // group base B = 2^(goff+J0) + HB uses twiddle (B << l) + (u >> (K-l)) at its
@@ -138,8 +138,8 @@ __device__ __forceinline__ void gs_reg(u64 (&v)[1 << K], const TW& tw, u32 B, u6
 //
 // Signed twiddles |w| <= (q-1)/2 (FpArS, the library's double tables): |h/q|
 // <= |y|/2, so with c = |y|/q and q < 2^50, |l| <= (c/16) q and
-//   M1 (needs |y| < 2^52, c <= 4)      :  |r| <= (1/2 + c/8) q,
-//   M2 (needs |y| < 2^53, c <= 8):           |r| <= (1 + c/8) q.
+//   M1 (needs |y| < 2^52, c <= 4):  |r| <= (1/2 + c/8) q,
+//   M2 (needs |y| < 2^53, c <= 8):  |r| <= (1 + c/8) q.
 // A value therefore stays exact while it is below 8q, whatever its round, and
 // a multiplied value falls back to 2q or less by itself. So the stages are
 // scheduled at compile time from the bound of their inputs (mul_bound,
