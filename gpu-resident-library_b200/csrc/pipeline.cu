@@ -475,6 +475,7 @@ static void commit(Plan& p, const HostTables& T, const std::vector<Op>& ops, cud
         for (int v = 0; v < 3; ++v) { p.job_off[k][v] = T.job_off[k][v]; p.job_cnt[k][v] = T.job_cnt[k][v]; }
     p.nops = (uint32_t)ops.size();
     p.ops = ops;
+    p.overwrites = -1;
     p.pairs_host = T.pairs;
 }
 
@@ -582,6 +583,7 @@ void rebind(Plan& p, uint32_t idx, const Op& op, const gfx::Context& c, cudaStre
     }
     p.pairs_host[idx] = P;
     p.ops[idx] = op;
+    p.overwrites = -1;
     k_set_pair<<<1, 1, 0, s>>>(p.d_pairs + idx, P);
 }
 
@@ -616,6 +618,31 @@ void apply_choice(Plan& p, int choice) {
     p.p3_form = (choice >> 3) & 3;
     if (p.p3_form > 2) p.p3_form = 0;
 }
+// Whether any output of the batch overlaps an input of it, the operation's own or
+// another's. Found once per set of buffers (a batch that is never timed asks at
+// every launch): inputs in order of their start, each with the furthest end up to
+// it, against the inputs that start before an output ends.
+bool overwrites_inputs(Plan& p) {
+    if (p.overwrites >= 0) return p.overwrites != 0;
+    const uintptr_t tower = sizeof(u64) << p.logn;
+    std::vector<std::pair<uintptr_t, uintptr_t>> in;
+    for (const Op& op : p.ops)
+        for (int k = 0; k < input_count(op.mode); ++k) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(op.in[k]);
+            in.push_back({a, a + op.L * tower});
+        }
+    std::sort(in.begin(), in.end());
+    for (size_t i = 1; i < in.size(); ++i) in[i].second = std::max(in[i].second, in[i - 1].second);
+    bool hit = false;
+    for (const Op& op : p.ops)
+        for (int k = 0; k < (op.mode == RESCALE ? 1 : 2); ++k) {
+            const uintptr_t a = reinterpret_cast<uintptr_t>(op.out[k]), b = a + output_towers(op) * tower;
+            const auto it = std::lower_bound(in.begin(), in.end(), std::make_pair(b, (uintptr_t)0));
+            hit = hit || (it != in.begin() && std::prev(it)->second > a);
+        }
+    p.overwrites = hit ? 1 : 0;
+    return hit;
+}
 }  // namespace
 
 void tune(Plan& p, cudaStream_t s, bool measure) {
@@ -634,21 +661,14 @@ void tune(Plan& p, cudaStream_t s, bool measure) {
     if (!measure) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
-    // Timing re-runs the batch, so a rescale must not write over an input: its
-    // own (in place) or another operation's. A batch with out-of-place rescales
-    // is timed like any other: without, 13 mixed operations at N = 2^14 kept the
-    // default key-product form (97 us where the tuned forms take 68; the whole step
-    // 402 -> 385 us). Rescales alone have no key product to choose a form for.
-    const size_t n = (size_t)1 << p.logn;
+    // Timing re-runs the batch, so none of its operations may write over an input.
+    // A batch with out-of-place rescales is timed like any other: without, 13 mixed
+    // operations at N = 2^14 kept the default key-product form (97 us where the
+    // tuned forms take 68; the whole step 402 -> 385 us). Rescales alone have no key
+    // product to choose a form for.
     bool keyed = false;
-    for (const Op& r : p.ops) {
-        keyed = keyed || r.mode != RESCALE;
-        if (r.mode != RESCALE) continue;
-        for (const Op& op : p.ops)
-            for (int k = 0; k < input_count(op.mode); ++k)
-                if (r.out[0] < op.in[k] + op.L * n && op.in[k] < r.out[0] + (r.L - 1) * n) return;
-    }
-    if (!keyed) return;
+    for (const Op& op : p.ops) keyed = keyed || op.mode != RESCALE;
+    if (!keyed || overwrites_inputs(p)) return;
     cudaEvent_t a, b;
     if (cudaEventCreate(&a) != cudaSuccess) return;
     if (cudaEventCreate(&b) != cudaSuccess) { cudaEventDestroy(a); return; }

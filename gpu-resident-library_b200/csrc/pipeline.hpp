@@ -48,6 +48,7 @@ struct Plan {
     unsigned mix = 0x1ff;              // bit k: phase k+1 as one launch over its interleaved job list
     int p3_form = 0;                   // 0 plain P3; 1, 2 warp-specialised (128 x 2 CTAs, 256 x 1 CTA)
     bool tuned = false;
+    int overwrites = -1;               // an output overlaps an input of the batch (-1: not looked at yet)
     // The plan's launches share the GPU with other streams' steps (the
     // server's rings run side by side): the autotuner, which times each
     // candidate alone, then leaves out the TMA form of the FP64 P5 rows,
@@ -91,8 +92,8 @@ cudaError_t launch(const Plan& p, cudaStream_t s, unsigned mask = 0x1ff);
 // candidate with CUDA events on `s` (one dimension at a time on the phases it
 // changes; two interleaved passes, best of three launches each; a candidate
 // wins only if 1.5% faster) and caching the winner. Timing re-runs the batch, so it is skipped (defaults
-// kept) when `measure` is false, while `s` is capturing a graph, or when a
-// rescale writes over an input of the batch (its own or another operation's).
+// kept) when `measure` is false, while `s` is capturing a graph, or when an
+// operation writes over an input of the batch (its own or another's).
 void tune(Plan& p, cudaStream_t s, bool measure = true);
 constexpr int MAC_MAX_DNUM = 16;
 // P5 forms: register prefetch with 128 threads x 4 words, the cp.async

@@ -306,7 +306,7 @@ int  gpufhe_plan_create(gpufhe_ctx* ctx, uint32_t nops, const gpufhe_op* ops, ui
 /* Launches the phase kernels for the whole batch on `stream` (kernel
  * launches only: capturable in a CUDA graph). The first launch outside
  * capture runs the autotuner, which re-runs the batch to time the candidate
- * schedules (skipped when a rescale writes over an input of the batch). */
+ * schedules (skipped when an operation writes over an input of the batch). */
 int  gpufhe_plan_launch(gpufhe_plan* plan, cudaStream_t stream);
 void gpufhe_plan_destroy(gpufhe_plan* plan);
 /* One phase (0..8 = P1..P9) only, for per-kernel timing. */
