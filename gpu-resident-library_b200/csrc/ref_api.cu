@@ -154,8 +154,11 @@ void rescale_component(u64* base, uint32_t towers, uint32_t n, const std::vector
     }
 }
 
-// Process-wide cache of packed twiddle tables for host-orchestrated helpers.
-struct TabEntry { Tw* f; Tw* i; u64 ninv, ninvp; };
+// Process-wide cache of twiddle tables for host-orchestrated helpers: packed
+// ones below 2^61, whose transforms let values grow to 8q, and split ones (w,
+// then the Shoup constants, n words each) for moduli up to 2^62, whose
+// transforms stay below 4q.
+struct TabEntry { Tw *f, *i; u64 *fs, *is; u64 ninv, ninvp; };
 std::mutex g_tab_mu;
 std::map<std::tuple<int, uint32_t, u64, u64>, TabEntry> g_tabs;
 
@@ -168,8 +171,20 @@ TabEntry tables_for(uint32_t n, u64 q, u64 root) {
     if (it != g_tabs.end()) return it->second;
     std::vector<Tw> f, iv;
     hm::twiddles(n, q, root, f, iv);
-    TabEntry e{dup_to_device(f), dup_to_device(iv), hm::invmod(n, q), 0};
+    TabEntry e{nullptr, nullptr, nullptr, nullptr, hm::invmod(n, q), 0};
     e.ninvp = hm::precon(e.ninv, q);
+    if (q < xf::PACKED_BELOW) {
+        e.f = dup_to_device(f);
+        e.i = dup_to_device(iv);
+    } else {
+        auto split = [&](const std::vector<Tw>& v) {
+            std::vector<u64> w(2 * (size_t)n);
+            for (uint32_t k = 0; k < n; ++k) { w[k] = v[k].w; w[n + k] = v[k].wp; }
+            return dup_to_device(w);
+        };
+        e.fs = split(f);
+        e.is = split(iv);
+    }
     g_tabs.emplace(key, e);
     return e;
 }
@@ -234,7 +249,8 @@ void launch_xform(u64* d, xf::Job* d_jobs, uint32_t towers, uint32_t n, const st
     std::vector<xf::Job> jobs(towers);
     for (uint32_t t = 0; t < towers; ++t) {
         TabEntry e = tables_for(n, mod[t], root[t]);
-        jobs[t] = xf::Job{d + (size_t)t * n, inverse ? e.i : e.f, nullptr, nullptr, mod[t], e.ninv, e.ninvp};
+        const u64* w = inverse ? e.is : e.fs;
+        jobs[t] = xf::Job{d + (size_t)t * n, inverse ? e.i : e.f, w, w ? w + n : nullptr, mod[t], e.ninv, e.ninvp};
     }
     ck(cudaMemcpy(d_jobs, jobs.data(), towers * sizeof(xf::Job), cudaMemcpyHostToDevice), "upload");
     ck(xf_launch_ntt(d_jobs, nullptr, (int)towers, hm::ilog2(n), inverse, 0), "transform");

@@ -13,8 +13,14 @@
 
 namespace xf {
 
+// Moduli of jobs with packed tables: their integer butterflies let values grow
+// to 8q (ntt::IntAr), which fits 64 bits below 2^61 only. Split tables take any
+// modulus below 2^62.
+constexpr u64 PACKED_BELOW = 1ull << 61;
+
 // One tower to transform in place. Twiddles either packed {w, wp} (library
-// tables) or split (two arrays, the reference's table layout). fp != 0 (only
+// tables, q < PACKED_BELOW) or split (two arrays, the reference's table
+// layout). fp != 0 (only
 // for q < 2^50) selects the FP64 arithmetic, with the signed double table twd
 // (twiddles in (-q/2, q/2)) or, when twd is null, the split w table converted
 // on load. Fields after scale_p default to zero (integer path) in brace
