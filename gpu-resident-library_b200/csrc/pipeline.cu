@@ -52,8 +52,7 @@ struct Variant {
         const PairDesc* pd = p.d_pairs;
         const uint2* J = p.d_jobs + p.job_off[k][PATH];
         auto run = [&](auto* kernel, unsigned grid, unsigned block, size_t smem) {
-            gfx::chain_launch(kernel, after, grid, block, smem, s, D, pd, J);
-            after = true;
+            if (gfx::chain_launch(kernel, after, grid, block, smem, s, D, pd, J) == cudaSuccess) after = true;
         };
         // a column kernel on wide tiles, or on narrow ones where those leave SMs idle
         const bool narrow = ntt::narrow_tiles<LOGN>(cnt, sm_count());
@@ -122,14 +121,15 @@ struct Launcher {
         const uint2* J = p.d_jobs + p.job_off[2][PATH];
         if (p.p3_form == 1) {
             const unsigned grid = std::min<unsigned>(ntiles, 2u * (unsigned)sm_count());
-            gfx::chain_launch(p3ws_modup_fwd_col<LOGN, PATH, 128, 2>, after, grid, P3WS<LOGN, 128>::NT,
-                              P3WS<LOGN, 128>::SMEM, s, p.dc, p.d_pairs, J, ntiles);
+            if (gfx::chain_launch(p3ws_modup_fwd_col<LOGN, PATH, 128, 2>, after, grid, P3WS<LOGN, 128>::NT,
+                                  P3WS<LOGN, 128>::SMEM, s, p.dc, p.d_pairs, J, ntiles) == cudaSuccess)
+                after = true;
         } else {
             const unsigned grid = std::min<unsigned>(ntiles, (unsigned)sm_count());
-            gfx::chain_launch(p3ws_modup_fwd_col<LOGN, PATH, 256, 1>, after, grid, P3WS<LOGN, 256>::NT,
-                              P3WS<LOGN, 256>::SMEM, s, p.dc, p.d_pairs, J, ntiles);
+            if (gfx::chain_launch(p3ws_modup_fwd_col<LOGN, PATH, 256, 1>, after, grid, P3WS<LOGN, 256>::NT,
+                                  P3WS<LOGN, 256>::SMEM, s, p.dc, p.d_pairs, J, ntiles) == cudaSuccess)
+                after = true;
         }
-        after = true;
     }
     // The integer forms of P5 over the first nint key-row jobs.
     static void launch_p5_int(const Plan& p, cudaStream_t s, uint32_t nint, bool& after) {
@@ -137,8 +137,9 @@ struct Launcher {
         const DevCtx& D = p.dc;
         const unsigned grid = nint * MAC_TILES;
         auto run = [&](auto* kernel, unsigned g, unsigned block, size_t smem) {
-            gfx::chain_launch(kernel, after, g, block, smem, s, D, p.d_pairs, p.d_mac_jobs, p.d_plist);
-            after = true;
+            if (gfx::chain_launch(kernel, after, g, block, smem, s, D, p.d_pairs, p.d_mac_jobs, p.d_plist) ==
+                cudaSuccess)
+                after = true;
         };
         if (p.p5_form == P5_TMA && mac_tma_ok(D.dnum))
             run(p5_mac_tma<LOGN>, nint * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum));
@@ -174,8 +175,9 @@ struct Launcher {
                 }
                 const uint4* fj = p.d_mac_jobs + p.job_off[4][1];
                 auto run = [&](auto* kernel, unsigned g, unsigned block, size_t smem) {
-                    gfx::chain_launch(kernel, after, g, block, smem, sf, D, p.d_pairs, fj, p.d_plist);
-                    after = !split;
+                    if (gfx::chain_launch(kernel, after, g, block, smem, sf, D, p.d_pairs, fj, p.d_plist) ==
+                            cudaSuccess && !split)
+                        after = true;
                 };
                 if (nfp && p.p5_fp_form == 2 && mac_tma_ok(D.dnum))
                     run(p5_mac_fp_tma<LOGN, 3>, nfp * ((1u << LOGN) / P5T_TILE), P5T_NT, p5t_smem((int)D.dnum, 3));

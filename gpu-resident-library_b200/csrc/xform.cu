@@ -15,14 +15,18 @@ cudaError_t launch_w(const xf::Job* jobs, const xf::Job& o, int njobs, bool inve
         cudaFuncSetAttribute(xf::k_fwd_row<LOGN, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
         cudaFuncSetAttribute(xf::k_inv_row<LOGN, SINGLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
     });
+    auto run = [&](auto* kernel, bool after, unsigned grid, unsigned block, size_t smem) {
+        return gfx::chain_launch(kernel, after, grid, block, smem, s, jobs, o) == cudaSuccess;
+    };
+    const unsigned col = njobs * G::COL_TILES, row = njobs * G::ROW_TILES;
     if (!inverse) {
-        xf::k_fwd_col<LOGN, SINGLE, W><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs, o);
-        return gfx::chain_launch(xf::k_fwd_row<LOGN, SINGLE>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
-                                 jobs, o);
+        if (run(xf::k_fwd_col<LOGN, SINGLE, W>, false, col, G::COL_THREADS, G::COL_SMEM))
+            run(xf::k_fwd_row<LOGN, SINGLE>, true, row, G::ROW_THREADS, G::ROW_SMEM);
+    } else {
+        if (run(xf::k_inv_row<LOGN, SINGLE>, false, row, G::ROW_THREADS, G::ROW_SMEM))
+            run(xf::k_inv_col<LOGN, SINGLE, W>, true, col, G::COL_THREADS, G::COL_SMEM);
     }
-    xf::k_inv_row<LOGN, SINGLE><<<njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s>>>(jobs, o);
-    return gfx::chain_launch(xf::k_inv_col<LOGN, SINGLE, W>, true, njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s,
-                             jobs, o);
+    return cudaGetLastError();   // of either launch
 }
 
 template <int LOGN, bool SINGLE>
@@ -41,9 +45,11 @@ cudaError_t launch_lift_w(const xf::Job* jobs, int njobs, cudaStream_t s) {
         cudaFuncSetAttribute(xf::k_fwd_col_lift<LOGN, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::COL_SMEM);
         cudaFuncSetAttribute(xf::k_fwd_row<LOGN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::ROW_SMEM);
     });
-    xf::k_fwd_col_lift<LOGN, W><<<njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s>>>(jobs);
-    return gfx::chain_launch(xf::k_fwd_row<LOGN, false>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s,
-                             jobs, xf::Job{});
+    if (gfx::chain_launch(xf::k_fwd_col_lift<LOGN, W>, false, njobs * G::COL_TILES, G::COL_THREADS, G::COL_SMEM, s,
+                          jobs) == cudaSuccess)
+        gfx::chain_launch(xf::k_fwd_row<LOGN, false>, true, njobs * G::ROW_TILES, G::ROW_THREADS, G::ROW_SMEM, s, jobs,
+                          xf::Job{});
+    return cudaGetLastError();   // of either launch
 }
 
 template <int LOGN>
