@@ -590,15 +590,31 @@ void rebind(Plan& p, uint32_t idx, const Op& op, const gfx::Context& c, cudaStre
 }
 
 namespace {
-uint64_t tune_key(const Plan& p) {
-    uint32_t cls = 0;
-    while ((1u << (cls + 1)) <= p.nops) ++cls;   // batch-size class: floor(log2(nops))
-    // hoisted rotations read their shared digits by an eval-slot gather, which
-    // favours other P5 forms than batches whose digits stream in order
-    bool hoisted = false;
-    for (const Op& op : p.ops) hoisted = hoisted || op.mode == HROT;
-    return (p.concurrent ? 1ull << 48 : 0ull) | ((uint64_t)p.logn << 40) | ((uint64_t)p.dc.dnum << 32) |
-           (hoisted ? 1ull << 16 : 0ull) | cls;
+// A schedule's place in the context's cache: the batch-size class, floor(log2) of
+// the number of operations with a key product (rescales have none, so they do
+// not set the key product's forms), beside what changes which forms win: rings
+// shared with other streams, hoisted rotations, rotations without products (the
+// P5 ring forms read their source blocks whole, the register forms gather them
+// word by word), and rescales, whose jobs take part in the choice of separate or
+// interleaved launches. So the order in which a program first launches its
+// batches does not matter: each kind is timed on its own kind.
+struct TuneKey {
+    uint64_t own;        // this batch's entry
+    uint64_t products;   // the entry of a batch of products of the same size
+};
+TuneKey tune_key(const Plan& p) {
+    uint32_t keyed = 0, cls = 0;
+    bool hoisted = false, plain = false, product = false;
+    for (const Op& op : p.ops) {
+        keyed += op.mode != RESCALE;
+        hoisted = hoisted || op.mode == HROT;
+        plain = plain || op.mode == ROT;
+        product = product || op.mode == EMR || op.mode == KS;
+    }
+    while ((2u << cls) <= (keyed ? keyed : p.nops)) ++cls;
+    const uint64_t base = (p.concurrent ? 1ull << 48 : 0ull) | ((uint64_t)p.logn << 40) |
+                          ((uint64_t)p.dc.dnum << 32) | (hoisted ? 1ull << 16 : 0ull) | cls;
+    return {base | (plain && !product ? 1ull << 17 : 0ull) | (keyed < p.nops ? 1ull << 18 : 0ull), base};
 }
 // choice: bits 0-1 = P5 form, bits 3-4 = P3 form (0 plain, 1 and 2
 // warp-specialised), bit 6 = P5 key rows of 50-bit Q towers on the FP64
@@ -650,16 +666,17 @@ bool overwrites_inputs(Plan& p) {
 void tune(Plan& p, cudaStream_t s, bool measure) {
     if (p.tuned || !p.nops || !p.ctx) return;
     const gfx::Context& c = *p.ctx;
-    const uint64_t key = tune_key(p);
+    const TuneKey key = tune_key(p);
     int choice = 0;
-    if (c.tuned_choice(key, choice)) {
+    if (c.tuned_choice(key.own, choice)) {
         apply_choice(p, choice);
         p.tuned = true;
         return;
     }
     // 4-word register P5 with FP64 Q rows, plain P3, interleaved paths
     constexpr int DEFAULT = P5_REG128 | 64 | (0x1ff << 8);
-    apply_choice(p, DEFAULT);
+    // until the batch is timed: the products' entry, else the default
+    apply_choice(p, c.tuned_choice(key.products, choice) ? choice : DEFAULT);
     if (!measure) return;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return;
@@ -727,7 +744,7 @@ void tune(Plan& p, cudaStream_t s, bool measure) {
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     apply_choice(p, cur);
-    c.set_tuned_choice(key, cur);
+    c.set_tuned_choice(key.own, cur);
     p.tuned = true;
 }
 

@@ -87,13 +87,15 @@ void build_plan_into(Plan& p, const gfx::Context& c, const std::vector<Op>& ops,
 // mask selects phases P1..P9 (bit k = phase k+1); 0x1ff runs the whole batch.
 cudaError_t launch(const Plan& p, cudaStream_t s, unsigned mask = 0x1ff);
 // Picks the launch schedule of `p` (P5 form; integer and FP64 transform
-// jobs as two launches or one interleaved launch): from the context's tuning cache when it holds
-// this shape (ring size, digits, batch-size class), else by timing every
-// candidate with CUDA events on `s` (one dimension at a time on the phases it
-// changes; two interleaved passes, best of three launches each; a candidate
-// wins only if 1.5% faster) and caching the winner. Timing re-runs the batch, so it is skipped (defaults
-// kept) when `measure` is false, while `s` is capturing a graph, or when an
-// operation writes over an input of the batch (its own or another's).
+// jobs as two launches or one interleaved launch): from the context's tuning
+// cache when it holds this shape (ring size, digits, batch-size class, kinds of
+// operation), else by timing every candidate with CUDA events on `s` (one
+// dimension at a time on the phases it changes; two interleaved passes, best of
+// three launches each; a candidate wins only if 1.5% faster) and caching the
+// winner. Timing re-runs the batch, so it is skipped (the schedule of a batch of
+// products of this size kept, or the default one) when `measure` is false, while
+// `s` is capturing a graph, or when an operation writes over an input of the
+// batch (its own or another's).
 void tune(Plan& p, cudaStream_t s, bool measure = true);
 constexpr int MAC_MAX_DNUM = 16;
 // P5 forms: register prefetch with 128 threads x 4 words, the cp.async
