@@ -17,18 +17,6 @@
 
 namespace gfx {
 
-// Whether a conversion of n sources below `below` (2^b) into a tower below 2^50
-// may take the FP64-quotient form (WrapConv in pipeline.cuh): the quotient's
-// error, in units, times q has to stay below 2^63.
-constexpr bool conv_wrap_ok(unsigned n, u64 below) {
-    int b = 0;
-    while (b < 63 && (1ull << b) < below) ++b;
-    double unit = 1.0;   // 2^(b - 54)
-    for (int k = 54; k < b; ++k) unit *= 2.0;
-    for (int k = b; k < 54; ++k) unit *= 0.5;
-    return b <= 61 && unit * (0.5 * n * (n + 1) + 2.5 * n) + 2048.0 + 64.0 < 8000.0;
-}
-
 constexpr int MAXQ = 48;     // Q towers
 constexpr int MAXP = 16;     // special primes
 constexpr int MAXQP = MAXQ + MAXP;

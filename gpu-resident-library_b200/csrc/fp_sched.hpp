@@ -1,7 +1,7 @@
-// Compile-time schedule of the FP64 transform rounds (FpArS in ntt.cuh): which
+// Compile-time schedules of the transform rounds in ntt.cuh: for FpArS, which
 // products take the even rounding and which values are normalised, from the
-// bounds of a round's inputs. Plain C++, so that the CPU check of the schedule
-// runs the same functions.
+// bounds of a round's inputs; for FpAr and IntAr, the stages that reduce. Plain
+// C++, so that the CPU checks of the schedules run the same functions.
 #pragma once
 
 #ifdef __CUDACC__
@@ -11,6 +11,9 @@
 #endif
 
 namespace ntt {
+
+constexpr double FP_M1 = 6755399441055744.0;    // 1.5 * 2^52
+constexpr double FP_M2 = 13510798882111488.0;   // 1.5 * 2^53
 
 // Bounds in units of q / 1024.
 constexpr int B_NORM = 514;     // a normalised value, |z| <= q/2 + 1
@@ -64,6 +67,17 @@ GFX_HD constexpr GsSched gs_sched(int K, int xin) {
     return S;
 }
 
+// FpAr (unsigned twiddles, every product by M2): whether all values are
+// normalised after local stage L of a forward / inverse round of K stages.
+GFX_HD constexpr bool fpar_ct_norm(int K, int L) { return L % 2 == 1 || L == K - 1; }
+GFX_HD constexpr bool fpar_gs_norm(int K, int L) { return (K - L) % 2 == 0 || L == 0; }
+
+// IntAr: whether a forward stage brings its untouched operand below 4q; whether
+// the pair at offset o of an inverse stage of half 2^s adds two sums (below 4q,
+// reduced) rather than two products (below 2q).
+GFX_HD constexpr bool int_ct_reduces(int L) { return L % 2 == 0; }
+GFX_HD constexpr bool int_gs_sums(int s, int o) { return s > 0 && (o >> (s > 0 ? s - 1 : 0) & 1) == 0; }
+
 GFX_HD constexpr int cmin(int a, int b) { return a < b ? a : b; }
 GFX_HD constexpr int cmax(int a, int b) { return a > b ? a : b; }
 
@@ -78,3 +92,13 @@ template <class AR>
 GFX_HD constexpr int inv_row_bound(int X0) { return AR::inv_out(4, AR::inv_out(4, X0)); }
 
 }  // namespace ntt
+
+namespace pl {
+
+// Bounds of the pipeline's transform inputs on the FP64 path: P1's tensor
+// products of canonical operands stay below 1.25q, P3's converted digits are
+// normalised, canonical or a sum of at most three signed products (0.63q each),
+// P8's prologue is normalised, U is canonical.
+constexpr int P1_IN = 1290, P3_IN = 1930, P8_IN = ntt::B_NORM, P6_IN = ntt::B_CANON;
+
+}  // namespace pl

@@ -130,7 +130,7 @@ __device__ __forceinline__ void gs_reg(u64 (&v)[1 << K], const TW& tw, u32 B, u6
 //     |l| <= |h| 2^-53 and |k - h/q| <= e + |h/q| 2^-53, e = 1/2 (M1) or 1 (M2).
 //   norm(z), |z| < 2^53: k = RN(z*qinv) by M1; z - k*q in [-q/2 - 1, q/2 + 1].
 //
-// Unsigned twiddles 0 <= w < q (FpArT<false>, tables converted on load): mul
+// Unsigned twiddles 0 <= w < q (FpAr, tables converted on load): mul
 // by M2 for |y| <= 4q gives |r| <= 2q. A round keeps every value normalised
 // at its start and end and normalises after every second stage: forward (CT)
 // values stay below 4.5q + 1 and multiplier inputs below 2.5q + 1; inverse
@@ -158,9 +158,6 @@ __device__ __forceinline__ void gs_reg(u64 (&v)[1 << K], const TW& tw, u32 B, u6
 // the row walks below, before -> after: 64 x 12 towers of 2^16, products and
 // inverse 650 -> 622 us, embedding 425 -> 415 us; phases of 128 products P1 355
 // -> 336, P2 270 -> 247, P3 1510 -> 1456, P4 1036 -> 1012 us.
-constexpr double FP_M1 = 6755399441055744.0;    // 1.5 * 2^52
-constexpr double FP_M2 = 13510798882111488.0;   // 1.5 * 2^53
-
 struct FpBase {
     using T = double;
     double q, qinv;
@@ -223,7 +220,7 @@ struct FpAr : FpBase {
                 y = __dsub_rn(xx, r);
             }
         }
-        if constexpr (L % 2 == 1 || L == K - 1) {
+        if constexpr (fpar_ct_norm(K, L)) {
 #pragma unroll
             for (int u = 0; u < (1 << K); ++u) v[u] = norm(v[u]);
         }
@@ -247,7 +244,7 @@ struct FpAr : FpBase {
                 y = mulq<true>(__dsub_rn(xx, yy), w);
             }
         }
-        if constexpr ((K - L) % 2 == 0 || L == 0) {
+        if constexpr (fpar_gs_norm(K, L)) {
 #pragma unroll
             for (int u = 0; u < (1 << K); ++u) v[u] = norm(v[u]);
         }
@@ -389,7 +386,7 @@ struct IntAr {
             for (int o = 0; o < half; ++o) {
                 u64& x = v[g * 2 * half + o];
                 u64& y = v[g * 2 * half + o + half];
-                const u64 xx = L % 2 == 0 ? csub(x, 2 * two_q) : x;
+                const u64 xx = int_ct_reduces(L) ? csub(x, 2 * two_q) : x;
                 const u64 r = shoup_lazy(y, t.w, t.wp, q);
                 x = xx + r;
                 y = xx - r + two_q;
@@ -408,7 +405,7 @@ struct IntAr {
                 const int i = g * 2 * half + o;
                 u64& x = v[i];
                 u64& y = v[i + half];
-                const bool sums = s > 0 && (o >> (s > 0 ? s - 1 : 0) & 1) == 0;   // both below 4q, else 2q
+                const bool sums = int_gs_sums(s, o);   // both below 4q, else 2q
                 const u64 d = x - y + (sums ? 2 * two_q : two_q);
                 x = sums ? csub(x + y, 2 * two_q) : x + y;
                 y = shoup_lazy(d, t.w, t.wp, q);

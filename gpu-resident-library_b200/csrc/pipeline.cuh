@@ -34,6 +34,7 @@
 #include <type_traits>
 
 #include "context.hpp"
+#include "conv_quot.hpp"
 #include "ntt.cuh"
 #include "pdl.cuh"
 
@@ -194,11 +195,6 @@ __device__ __forceinline__ u64 conv_reduce(u64 lo, u64 hi, const ModC& m, u32 mo
     return mont ? redc_lazy(lo, hi, m) : barrett_lazy(lo, hi, m.q, m.mu_lo, m.mu_hi);
 }
 
-// One term of a basis conversion in shared memory: the constant, and its ratio
-// to the target modulus (quotient form below) or its value as a double (P3's
-// FP64 products).
-struct __align__(16) ConvTerm { u64 c; double f; };
-
 // lo/hi[b][j] += sum_{t < nterms} base[t * stride + e[b] + j] * coef[t].c (128-bit).
 template <int VB>
 __device__ __forceinline__ void mac_terms(u64 (&lo)[VB][2], u64 (&hi)[VB][2], const u64* base, size_t stride,
@@ -223,11 +219,7 @@ __device__ __forceinline__ void mac_terms(u64 (&lo)[VB][2], u64 (&hi)[VB][2], co
     }
 }
 
-// Bounds of the transforms' inputs on the FP64 path (units of q / 1024, see
-// ntt.cuh): P1's tensor products of canonical operands stay below 1.25q, P3's
-// converted digits are normalised, canonical or a sum of at most three signed
-// products (0.63q each), P8's prologue is normalised, U is canonical.
-constexpr int P1_IN = 1290, P3_IN = 1930, P8_IN = ntt::B_NORM, P6_IN = ntt::B_CANON;
+// Bounds between the two passes, from the inputs' (P1_IN .. P6_IN).
 template <bool FP>
 __host__ __device__ constexpr int inv_bound(int x0) {
     return ntt::inv_row_bound<std::conditional_t<FP, ntt::FpArS, ntt::IntAr>>(x0);
@@ -237,32 +229,16 @@ __host__ __device__ constexpr int fwd_bound(int A, int x0) {
     return ntt::fwd_col_bound<std::conditional_t<FP, ntt::FpArS, ntt::IntAr>>(A, x0);
 }
 
-// Basis conversion into a tower q < 2^50 by an FP64 quotient (P8, where
-// DevCtx::wrap_down). sum_t x_t c_t mod q needs only
-//   r1 = sum_t x_t c_t - K q   (mod 2^64),   K near S = sum_t x_t (c_t / q),
-// as long as r1 fits 64 bits: low 64-bit products on the integer pipes (one
-// wide and two narrow multiplies) and one FMA per term for S on the FP64 pipe.
-// The 128-bit multiply-add of mac_terms takes four wide multiplies and
-// carries (22 issue cycles a term on one scheduler, measured, a wide multiply
-// five of them) and its Montgomery or Barrett step thirty more. Constants are
-// signed, |c_t / q| <= 1/2. Sources below 2^b are rounded to doubles, so S
-// sums n terms with an error of at most 2^(b-54) (n (n+1) / 2 + 5 n / 2); K is
-// S rounded to a multiple of 2^12 (error 2^11). Where conv_wrap_ok admits (n,
-// b), |r1| < 2^13 q < 2^63, and a second step, K2 = r1 / q rounded, leaves
-// |r| <= q/2 + 1, which the transform takes as it is. Words become doubles by
-// the conversion instruction: two FP64 additions of biased halves took four
-// issue slots (P8 of 128 products 960 -> 912 us). Measured before that: P8 of 128
-// products (N = 2^16, four terms) 1078 -> 966 us, of 48 rotations 492 -> 431 us,
-// of 13 mixed operations (N = 2^14, nine terms) 72 -> 65 us. In P3 and P7 the
-// same form gained nothing: their 50-bit sources already go to exact FP64
-// products, and P7's one conversion per component is not what it waits for.
-// ConvTerm of the residue c (canonical mod q), negated when NEG.
-template <bool NEG>
-__device__ __forceinline__ ConvTerm conv_term(u64 c, const ModC& m) {
-    long long v = c > (m.q >> 1) ? (long long)c - (long long)m.q : (long long)c;
-    if (NEG) v = -v;
-    return ConvTerm{(u64)v, __dmul_rn((double)v, qinv_of(m))};
-}
+// Quotient form of a conversion (conv_quot.hpp; P8, where DevCtx::wrap_down).
+// The 128-bit multiply-add of mac_terms takes four wide multiplies and carries
+// (22 issue cycles a term on one scheduler, measured, a wide multiply five of
+// them) and its Montgomery or Barrett step thirty more; this form one wide and
+// two narrow multiplies and an FMA. Measured, before the conversion instruction
+// (see quot_term): P8 of 128 products (N = 2^16, four terms) 1078 -> 966 us, of 48
+// rotations 492 -> 431 us, of 13 mixed operations (N = 2^14, nine terms) 72 -> 65
+// us. In P3 and P7 the same form gained nothing: their 50-bit sources already go
+// to exact FP64 products, and P7's one conversion per component is not what it
+// waits for.
 // lo[b][j] += sum_t x c_t mod 2^64, s[b][j] += sum_t x f_t.
 template <int VB>
 __device__ __forceinline__ void quot_terms(u64 (&lo)[VB][2], double (&s)[VB][2], const u64* base, size_t stride,
@@ -282,29 +258,12 @@ __device__ __forceinline__ void quot_terms(u64 (&lo)[VB][2], double (&s)[VB][2],
                 for (int b = 0; b < VB; ++b)
 #pragma unroll
                     for (int j = 0; j < 2; ++j) {
-                        const u64 x = j ? xv[tt][b].y : xv[tt][b].x;
-                        lo[b][j] += x * c.c;
-                        s[b][j] = __fma_rn(__ull2double_rn(x), c.f, s[b][j]);
+                        quot_term(lo[b][j], s[b][j], j ? xv[tt][b].y : xv[tt][b].x, c);
                     }
             }
     }
 }
-struct WrapConv {
-    u64 q;
-    double qinv;
-    __device__ __forceinline__ explicit WrapConv(const ModC& m) : q(m.q), qinv(qinv_of(m)) {}
-    // r = lo - K q, |r| <= q/2 + 1
-    __device__ __forceinline__ long long finish(u64 lo, double s) const {
-        const long long k = __double_as_longlong(__dadd_rn(s, 0x1.8p64)) - 0x43F8000000000000ll;
-        const u64 r1 = lo - (u64)k * (q << 12);
-        const double rd = __ll2double_rn((long long)r1);
-        const int k2 = __double2loint(__fma_rn(rd, qinv, ntt::FP_M1));
-        return (long long)(r1 - (u64)(long long)k2 * q);
-    }
-    __device__ __forceinline__ double finish_d(u64 lo, double s) const {
-        return __dsub_rn(__longlong_as_double(finish(lo, s) + 0x4338000000000000ll), ntt::FP_M1);
-    }
-};
+
 // ------------------------------------------------------------------ P1
 template <int LOGN, bool FP>
 __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc* __restrict__ pairs, const uint2 jb,
@@ -1859,7 +1818,7 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
     // makes -q_l s2 one (mod q_i); ci[K] holds s2, ci[0..K) the negated terms.
     if constexpr (FP) {
         if (D.wrap_down) {
-            const WrapConv wc(m);
+            const WrapConv wc{m.q, qinv_of(m)};
 #pragma unroll 1
             for (int k0 = 0; k0 < CS::PER; k0 += P8_VB) {
                 int r[P8_VB], cl[P8_VB];
@@ -1882,8 +1841,8 @@ __device__ __forceinline__ void p8_body(const DevCtx& D, const PairDesc& P, u32 
                         if constexpr (MODE == EMR || MODE == RESCALE) {
                             const ConvTerm t = ci[K];
                             const u64 x = j ? xr[b].y : xr[b].x;
-                            lo[b][j] += x * t.c + (x > half ? 1ull : 0ull);
-                            sq[b][j] = __fma_rn(__ull2double_rn(x), t.f, sq[b][j]);
+                            quot_term(lo[b][j], sq[b][j], x, t);
+                            lo[b][j] += x > half ? 1ull : 0ull;
                         }
                         v[j] = wc.finish_d(lo[b][j], sq[b][j]);
                     }
@@ -1961,13 +1920,13 @@ __device__ __forceinline__ void p8_moddown_fwd_col_body(const DevCtx& D, const P
         const u64 cm = P.mode == EMR ? D.lvl[P.L].ps1[i] : D.pinv[i];
         u64 v = mulmod(D.phatmodq[threadIdx.x * D.fullQ + i], cm, mi);
         if (quot) {
-            ci[threadIdx.x] = conv_term<true>(v, mi);
+            ci[threadIdx.x] = conv_term<true>(v, mi.q, qinv_of(mi));
         } else {
             if (D.mont_down) v = mulmod(v, r_mod(mi), mi);
             ci[threadIdx.x] = ConvTerm{v, 0.0};
         }
     } else if (quot && threadIdx.x == D.K && (P.mode == EMR || P.mode == RESCALE)) {
-        ci[D.K] = conv_term<false>(D.lvl[P.L].s2[i], D.mod[i]);
+        ci[D.K] = conv_term<false>(D.lvl[P.L].s2[i], D.mod[i].q, qinv_of(D.mod[i]));
     }
     __syncthreads();
     if (P.mode == EMR) p8_body<LOGN, W, EMR, FP>(D, P, c, i, c0, sm, ci);

@@ -17,7 +17,7 @@
 
 typedef unsigned __int128 u128;
 typedef uint64_t u64;
-static const double M1 = 6755399441055744.0, M2 = 13510798882111488.0;
+static const double M1 = ntt::FP_M1, M2 = ntt::FP_M2;
 static const double TWO52 = 4503599627370496.0, TWO53 = 9007199254740992.0;
 static double q, qinv;
 static u64 Q;
@@ -118,7 +118,7 @@ int main(int argc, char** argv) {
     const u64 mods[] = {1125899906826241ull, 1125899903827969ull, 562949955125249ull, 1073872897ull};
     const long trials = argc > 1 ? atol(argv[1]) : 2000;
     // input bounds of the kernels: normalised, canonical, tensor products, sums of three converted products
-    const int starts[] = {ntt::B_NORM, ntt::B_CANON, 1290, 1930};
+    const int starts[] = {pl::P8_IN, pl::P6_IN, pl::P1_IN, pl::P3_IN};
     std::set<int> fwd[5], inv[5];
     for (int x0 : starts)
         for (int A = 1; A <= 8; ++A) {

@@ -1,6 +1,6 @@
 """The pipeline's conversions at the edges of their forms: special primes and
 digit widths on both sides of the bound that allows the FP64-quotient form
-(conv_wrap_ok in csrc/context.hpp), tower widths from 30 to 60 bits, inputs at
+(conv_wrap_ok in csrc/conv_quot.hpp), tower widths from 30 to 60 bits, inputs at
 0 and q - 1. Products, rotations, keyswitches and rescales equal the oracle
 bit for bit in separate and in interleaved launches."""
 import numpy as np
@@ -24,14 +24,17 @@ def residues(rng, mods, n, edge):
 @pytest.mark.parametrize("n,bits,K,alpha,pbits", [
     (1024, (60, 50, 50, 50, 50), 1, 1, 60),
     (2048, (60, 50, 50, 50, 50, 50, 50), 3, 3, 60),
-    (1024, (60,) + (50,) * 9, 8, 8, 60),             # nine terms: the widest that fits at 60 bits
-    (1024, (60,) + (50,) * 5, 9, 5, 60),             # ten terms: the 128-bit form
+    (1024, (60,) + (50,) * 9, 8, 8, 60),             # nine terms
+    (1024, (60,) + (50,) * 5, 9, 5, 60),             # ten terms: the widest that fits at 60 bits
+    (1024, (60,) + (50,) * 5, 10, 5, 60),            # eleven: the 128-bit form
     (1024, (60,) + (50,) * 5, 13, 6, 60),
     (1024, (60,) + (50,) * 5, 12, 6, 50),            # 50-bit special primes
     (1024, (50, 50, 50, 50), 2, 2, 60),
     (1024, (60, 30, 40, 30, 45, 49), 2, 3, 60),      # narrow towers
     (1024, (60, 55, 55, 50, 55), 2, 2, 60),
     (4096, (50, 60, 50, 60, 50), 4, 4, 55),
+    (1024, (61,) + (50,) * 5, 6, 5, 61),             # seven terms: the widest that fits at 61 bits
+    (1024, (61,) + (50,) * 5, 7, 5, 61),             # eight: the 128-bit form
     (1024, (61, 61, 50, 61), 2, 2, 61),              # the widest towers: 8q just below 2^64
 ])
 def test_conversion_forms(n, bits, K, alpha, pbits):
