@@ -578,17 +578,14 @@ __device__ __forceinline__ void row_round(const AR& ar, const TW& tw, u32 R0, LD
     for (int u = 0; u < (1 << K); ++u) st(rl, cb + (u << SH), v[u]);
 }
 
-template <int KMAX, int J0>
-struct RowK { static constexpr int K = cmin(KMAX, 8 - J0); };
-
-// Forward row pass: stages A..A+7, rounds of KMAX. The first round reads a
+// Forward row pass: stages A..A+7, two rounds of four. The first round reads a
 // forward column pass's words as the policy's values (bounded by BIN) with
 // `ld` directly; the last round writes shared memory, and the caller then
 // reads the tile row-contiguously (coalesced) and converts each word with
 // ar.final_canon or ar.final_2q.
-template <int A, int RB, int NT, int KMAX, int J0, int BIN, class AR, class TW, class LD>
+template <int A, int RB, int NT, int J0, int BIN, class AR, class TW, class LD>
 __device__ __forceinline__ void fwd_row_rounds(u64* sm, const TW& tw, u32 R0, const AR& ar, LD&& ld) {
-    constexpr int K = RowK<KMAX, J0>::K;
+    constexpr int K = 4;
     constexpr bool LAST = (J0 + K == 8);
     constexpr int STR = 256 + 16;
     using T = typename AR::T;
@@ -597,17 +594,16 @@ __device__ __forceinline__ void fwd_row_rounds(u64* sm, const TW& tw, u32 R0, co
     if constexpr (J0 == 0) row_round<A, RB, NT, J0, K, true, BIN, LAST>(ar, tw, R0, ld, sst);
     else row_round<A, RB, NT, J0, K, true, BIN, LAST>(ar, tw, R0, sld, sst);
     __syncwarp();
-    if constexpr (!LAST) fwd_row_rounds<A, RB, NT, KMAX, J0 + K, AR::fwd_out(K, BIN)>(sm, tw, R0, ar, ld);
+    if constexpr (!LAST) fwd_row_rounds<A, RB, NT, J0 + K, AR::fwd_out(K, BIN)>(sm, tw, R0, ar, ld);
 }
 
 // Inverse row pass: GS stages A+7..A. Input is staged into shared memory
 // (row-contiguous, coalesced) by the caller as the policy's words (bounded by
 // BIN); the last round stores the policy's own words via `st`, for a
 // following column pass.
-template <int A, int RB, int NT, int KMAX, int JE, int BIN, class AR, class TW, class ST>
+template <int A, int RB, int NT, int JE, int BIN, class AR, class TW, class ST>
 __device__ __forceinline__ void inv_row_rounds(u64* sm, const TW& tw, u32 R0, const AR& ar, ST&& st) {
-    constexpr int J0 = ((JE - 1) / KMAX) * KMAX;
-    constexpr int K = JE - J0;
+    constexpr int K = 4, J0 = JE - K;
     constexpr bool LAST = (J0 == 0);
     constexpr int STR = 256 + 16;
     using T = typename AR::T;
@@ -618,7 +614,7 @@ __device__ __forceinline__ void inv_row_rounds(u64* sm, const TW& tw, u32 R0, co
     else {
         row_round<A, RB, NT, J0, K, false, BIN, false>(ar, tw, R0, sld, sst);
         __syncwarp();
-        inv_row_rounds<A, RB, NT, KMAX, J0, AR::inv_out(K, BIN)>(sm, tw, R0, ar, st);
+        inv_row_rounds<A, RB, NT, J0, AR::inv_out(K, BIN)>(sm, tw, R0, ar, st);
     }
 }
 

@@ -299,7 +299,7 @@ __device__ __forceinline__ void p1_inv_row_body(const DevCtx& D, const PairDesc*
     }
     __syncwarp();
     auto st = [&](int rl, int c, u64 v) { X[rl * 256 + c] = v; };
-    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, P1_IN>(sm, twi_of<FP>(D, i, LOGN), R0, ar, st);
+    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 8, P1_IN>(sm, twi_of<FP>(D, i, LOGN), R0, ar, st);
 }
 
 template <int LOGN, int PATH>
@@ -585,7 +585,7 @@ __device__ __forceinline__ void p4_modup_fwd_row_body(const DevCtx& D, const Pai
     u64* Y = slot_ptr(P, w.Y + p * QlP + i, LOGN) + (size_t)R0 * 256;
     const auto ar = ar_of<FP>(m);
     auto ld = [&](int rl, int c) { return ar.unbits(Y[rl * 256 + c]); };
-    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, fwd_bound<FP>(G::A, P3_IN)>(sm, twf_of<FP>(D, qp, LOGN), R0,
+    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 0, fwd_bound<FP>(G::A, P3_IN)>(sm, twf_of<FP>(D, qp, LOGN), R0,
                                                                                        ar, ld);
     ntt::row_tile_walk<G::RB, G::ROW_THREADS>([&](int e, int si) { Y[e] = ar.final_2q(sm[si]); });
 }
@@ -1659,7 +1659,7 @@ __device__ __forceinline__ void p6_moddown_inv_row_body(const DevCtx& D, const P
                                                [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in_canon(v)); });
     __syncwarp();
     auto st = [&](int rl, int cc, u64 v) { X[rl * 256 + cc] = v; };
-    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, P6_IN>(sm, twi_of<FP>(D, qp, LOGN), R0, ar, st);
+    ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 8, P6_IN>(sm, twi_of<FP>(D, qp, LOGN), R0, ar, st);
 }
 
 template <int LOGN, int PATH>
@@ -1959,7 +1959,7 @@ __device__ __forceinline__ void p9_final_fwd_row_body(const DevCtx& D, const Pai
     const u64* Z = slot_ptr(P, w.Z + c * L + i, LOGN) + tile0;
     const auto ar = ar_of<FP>(m);
     auto ld = [&](int rl, int cc) { return ar.unbits(Z[rl * 256 + cc]); };
-    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, fwd_bound<FP>(G::A, P8_IN)>(sm, twf_of<FP>(D, i, LOGN), R0,
+    ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 0, fwd_bound<FP>(G::A, P8_IN)>(sm, twf_of<FP>(D, i, LOGN), R0,
                                                                                        ar, ld);
     const size_t o = ((size_t)i << LOGN) + tile0;
     u64* out = P.out[c] + o;

@@ -131,7 +131,7 @@ k_fwd_row(const Job* __restrict__ arr, const Job one) {
     with_path(j, [&](const auto& ar, const auto& tw) {
         using AR = std::decay_t<decltype(ar)>;
         auto ld = [&](int rl, int c) { return ar.unbits(x[rl * 256 + c]); };
-        ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 0, ntt::fwd_col_bound<AR>(G::A, COL_IN)>(sm, tw, R0, ar,
+        ntt::fwd_row_rounds<G::A, G::RB, G::ROW_THREADS, 0, ntt::fwd_col_bound<AR>(G::A, COL_IN)>(sm, tw, R0, ar,
                                                                                                      ld);
         ntt::row_tile_walk<G::RB, G::ROW_THREADS>([&](int e, int si) { x[e] = ar.final_canon(sm[si]); });
     });
@@ -152,7 +152,7 @@ k_inv_row(const Job* __restrict__ arr, const Job one) {
         ntt::row_tile_stage<G::RB, G::ROW_THREADS>([&](int e) { return x[e]; },
                                                    [&](int, int si, u64 v) { sm[si] = ar.bits(ar.in(v)); });
         __syncwarp();
-        ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 4, 8, ntt::B_NORM>(sm, tw, R0, ar, st);
+        ntt::inv_row_rounds<G::A, G::RB, G::ROW_THREADS, 8, ntt::B_NORM>(sm, tw, R0, ar, st);
     });
 }
 
